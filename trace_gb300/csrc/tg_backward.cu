@@ -7,6 +7,8 @@ namespace tg {
 
 TG_BACKWARD_ENTRY(1)
 TG_BACKWARD_ENTRY(2)
+TG_BACKWARD_MULTI_ENTRY(1)
+TG_BACKWARD_MULTI_ENTRY(2)
 
 void launch_backward_multi(const BackItem* items, int n, int64_t blocks, int K,
                            int dlen_kind, int pen, int fh, int comp, cudaStream_t st) {
@@ -14,8 +16,7 @@ void launch_backward_multi(const BackItem* items, int n, int64_t blocks, int K,
     case 1: launch_backward_multi_k1(items, n, blocks, dlen_kind, pen, fh, comp, st); break;
     case 2: launch_backward_multi_k2(items, n, blocks, dlen_kind, pen, fh, comp, st); break;
     case 4: launch_backward_multi_k4(items, n, blocks, dlen_kind, pen, fh, comp, st); break;
-    case 8: launch_backward_multi_k8(items, n, blocks, dlen_kind, pen, fh, comp, st); break;
-    default: launch_backward_multi_k16(items, n, blocks, dlen_kind, pen, fh, comp, st); break;
+    default: launch_backward_multi_k8(items, n, blocks, dlen_kind, pen, fh, comp, st); break;
   }
 }
 

@@ -1,5 +1,8 @@
 // Backprojection (pixel-driven) with the algorithms' UpdateRecon fused into
-// its epilogue.
+// its epilogue: exact mode, plans without the tile-staged forward, fewer than
+// 8 slices per pass with FP32 operands, compensated sums and the
+// allocation-free entry point. The other plans' runs on the tensor cores
+// (tg_backward_mma.cuh).
 //
 // One thread per pixel, one warp per 32-pixel tile (8x4 by default; 16x2
 // or 4x8 as the plan chooses), eight tiles per block.
@@ -388,25 +391,26 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<K, COMP>()))
                                               s_coef);
 }
 
-// Multi-plan launches for plans with 16-bit fixed-point lengths: their
-// backward matrix holds u16 codes, or IEEE halves with half gathers.
+// Multi-plan launches for plans with 16-bit fixed-point lengths: compensated
+// sums (backward matrix u16 codes, or IEEE halves with half gathers), or FP32
+// operands at fewer than 8 slices per pass; the rest is tg_backward_mma.cuh's.
 template <int K>
 void back_multi(const BackItem* items, int n, int64_t blocks, int dlen_kind, int pen,
                 int fh, int comp, cudaStream_t st) {
-#define TG_BM(LKK, PN, FHH, CP) \
-  k_backward_multi<K, LKK, PN, FHH, CP><<<(unsigned)blocks, kBlock, 0, st>>>(items, n)
-  constexpr bool kComp = K <= 8;  // compensated sums: up to 8 slices per pass
-#define TG_BM_PC(LKK, FHH)                                                               \
+#define TG_BM(LKK, FHH, CP)                                                              \
   do {                                                                                   \
-    if (pen) { if (kComp && comp) TG_BM(LKK, true, FHH, kComp); else TG_BM(LKK, true, FHH, false); } \
-    else { if (kComp && comp) TG_BM(LKK, false, FHH, kComp); else TG_BM(LKK, false, FHH, false); }   \
+    if (pen)                                                                             \
+      k_backward_multi<K, LKK, true, FHH, CP><<<(unsigned)blocks, kBlock, 0, st>>>(items, n);  \
+    else                                                                                 \
+      k_backward_multi<K, LKK, false, FHH, CP><<<(unsigned)blocks, kBlock, 0, st>>>(items, n); \
   } while (0)
-  if (dlen_kind == LK_F16) {
-    if (fh) TG_BM_PC(LK_F16, true); else TG_BM_PC(LK_F16, false);
+  if (!comp) {
+    if constexpr (K < 8) TG_BM(LK_U16, false, false);
+  } else if (dlen_kind == LK_F16) {
+    if (fh) TG_BM(LK_F16, true, true); else TG_BM(LK_F16, false, true);
   } else {
-    TG_BM_PC(LK_U16, false);
+    TG_BM(LK_U16, false, true);
   }
-#undef TG_BM_PC
 #undef TG_BM
 }
 
@@ -429,7 +433,11 @@ void back_launch(const IterArgs& A, int batch, const float* cur, float* next,
       if (pen) TG_BACK(false, true, false, kComp); else TG_BACK(false, false, false, kComp);
     }
   } else if (A.half_factors) {
-    if (pen) TG_BACK(false, true, true, false); else TG_BACK(false, false, true, false);
+    // float lengths only: half factors with 16-bit lengths are
+    // tg_backward_mma.cuh's
+    if constexpr (LK == LK_F32) {
+      if (pen) TG_BACK(false, true, true, false); else TG_BACK(false, false, true, false);
+    }
   } else {
     if (pen) TG_BACK(false, true, false, false); else TG_BACK(false, false, false, false);
   }
@@ -450,13 +458,15 @@ void back_kind(const IterArgs& A, int batch, const float* cur, float* next,
 }  // namespace
 
 // Backprojection launches for one K, each K compiled in its own translation
-// unit (tg_backward*.cu) so the template instances build in parallel.
+// unit (tg_backward*.cu) so the template instances build in parallel; the
+// multi-plan launches serve up to 8 slices per pass.
 #define TG_BACKWARD_ENTRY(KK)                                                           \
   void launch_backward_k##KK(const IterArgs& A, int batch, const float* recon_cur,     \
                              float* recon_next, const float* upd, float* rep_num,      \
                              int epi, cudaStream_t st) {                               \
     back_kind<KK>(A, batch, recon_cur, recon_next, upd, rep_num, epi, st);             \
-  }                                                                                     \
+  }
+#define TG_BACKWARD_MULTI_ENTRY(KK)                                                     \
   void launch_backward_multi_k##KK(const BackItem* items, int n, int64_t blocks,       \
                                    int dlen_kind, int pen, int fh, int comp,            \
                                    cudaStream_t st) {                                   \

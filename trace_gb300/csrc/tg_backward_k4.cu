@@ -4,5 +4,6 @@
 namespace tg {
 
 TG_BACKWARD_ENTRY(4)
+TG_BACKWARD_MULTI_ENTRY(4)
 
 }  // namespace tg

@@ -4,5 +4,6 @@
 namespace tg {
 
 TG_BACKWARD_ENTRY(8)
+TG_BACKWARD_MULTI_ENTRY(8)
 
 }  // namespace tg

@@ -212,6 +212,19 @@ __device__ __forceinline__ int window_c0(float4 coef, float xf, float yf) {
   return __float_as_int(__fadd_rn(v, 12582912.0f)) - 0x4B400000;
 }
 
+// window_c0 with its bias left in.
+constexpr int kWindowBias = 0x4B400000;
+__device__ __forceinline__ int window_bits(float4 cf, float xf, float yf) {
+  return window_c0(cf, xf, yf) + kWindowBias;
+}
+
+// The smallest window_bits over the nx x ny pixels from (x0, y0): window_c0
+// is monotone in x and in y, so it is that of a corner.
+__device__ __forceinline__ int window_low(float4 cf, int x0, int y0, int nx, int ny) {
+  return window_bits(cf, (float)(cf.x < 0.f ? x0 + nx - 1 : x0),
+                     (float)(cf.y < 0.f ? y0 + ny - 1 : y0));
+}
+
 // Backward-matrix pair index (two slots) of angle a, tile t, lane l: angles
 // in groups of four per lane, so one 16-byte load brings four angles.
 __device__ __forceinline__ int64_t dense_pair(int ntiles, int a, int t, int l) {

@@ -28,6 +28,11 @@ struct MatrixDev {
   // and (a, window_c0 + 1) through the pixel
   const void* dlen;
   const float4* wcoef; // [P4] window coefficients {-sin, cos, D, 0}
+  // tensor-core backprojection: per angle quad and 4x4 pixel tile (tiles4 per
+  // row and column) 16 words, of pixels 0, 8, 1, 9, ..., 7, 15 of the tile;
+  // byte a & 3 of a word is the pixel's place_byte at angle a
+  const uint32_t* place;
+  int tiles4;
   // segments outside their pixel's two-column window (rare: the reference's
   // tracer puts a stray segment far from its ray at some near-vertical
   // angles): per pixel tile t, entries exc[exc_first[t] .. exc_first[t+1]) =
@@ -108,9 +113,58 @@ enum FwdOut { FWD_SIRT = 0, FWD_RATIO = 1, FWD_SIM = 2 };
 // What the backward kernel does with its per-pixel sums.
 enum BackEpi { EPI_UPDATE = 0, EPI_REPLICA = 1 };
 
+// Per-ray factors as the tensor-core backprojection (tg_backward_mma.cuh)
+// reads them: units of U = 8, 16 or 32 slices, each [P4][RP][U] floats or
+// halves with kRayPad zero columns before column 0 of an angle and twice as
+// many after the last (windows may start and end outside the detector).
+// flags[b] != 0: slice batch b holds a non-finite factor on a ray with
+// segments (reset by the batch's forward launch, raised by its finish).
+constexpr int kRayPad = 8;
+// Float factors of plans with f16 lengths are also kept as two halves each,
+// [P4][RP][2][U] (high parts, then low), scaled per slice by
+// split_scale(fmax[slice]); fmax: bits of the slice's largest |factor|,
+// reset and raised as the flags are.
+struct FactorDev {
+  void* base;
+  __half* split;
+  unsigned* fmax;
+  int64_t unit_elems;  // P4 * RP * U
+  int U, RP;
+  int ring;            // units held; unit u is at u % ring
+  int* flags;
+  int nflags;          // slice batches
+  int blocks_x;        // 16 x 8 pixel blocks per row
+};
+// at least the 21 columns that a block stages
+inline int factor_row(int C) { return C + 3 * kRayPad; }
+inline int64_t mma_regions(int C) { return (int64_t)((C + 15) / 16) * ((C + 7) / 8); }
+
+// The power of two that takes a largest |factor| (its float bits) to [2^13,
+// 2^14): 1 for zero; kept finite, with a finite inverse, at the ends.
+__host__ __device__ __forceinline__ float split_scale(unsigned bits) {
+  const int e = (int)(bits >> 23);  // biased exponent
+  if (e == 0) return 1.f;
+  const int b = 127 + 13 - (e - 127);  // biased exponent of the scale
+  const unsigned u = (unsigned)(b < 1 ? 1 : b > 253 ? 253 : b) << 23;
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(u);
+#else
+  float f;
+  memcpy(&f, &u, 4);
+  return f;
+#endif
+}
+
+// Element of column c, angle a, slice su of the unit at unit_base.
+__device__ __forceinline__ int64_t factor_at(int64_t unit_base, int RP, int U, int a, int c,
+                                             int su) {
+  return unit_base + ((int64_t)a * RP + c + kRayPad) * U + su;
+}
+
 struct IterArgs {
   DevGeom G;
   MatrixDev M;
+  FactorDev F;        // tensor-core backprojection (U = 0: the scalar kernels)
   int K;              // slices per pass
   int S;              // sinogram slices
   int alg;            // 0..3
@@ -141,6 +195,8 @@ struct FwdItem {
   TileMatrixDev T;
   const float* recon;   // the batch's reconstruction slots
   float* part;          // the plan's partial-sum slots
+  int* flag;            // the batch's non-finite flag (nullptr: none), reset here
+  unsigned* fmax;       // and its slices' largest factors (nullptr: none)
   int g;
   float inv_scale;
   int64_t first;
@@ -164,7 +220,10 @@ struct FinItem {
   const float* ra2;
   const float* part;
   const float* sino;    // the batch's sinogram rows
-  float* out;           // per-ray factors
+  float* out;           // per-ray factors [rays][K], or F when F.U != 0
+  FactorDev F;
+  int batch, C;
+  int P4, S;            // launch_split_factors_multi
   int64_t nrays;
   int64_t first;        // 256 rays a block
   int out_mode;
@@ -173,6 +232,7 @@ struct FinItem {
 struct BackItem {
   IterArgs A;
   int batch;
+  int nunits;           // tensor-core backprojection: units of the plan
   const float* cur;
   float* next;
   const float* upd;
@@ -233,6 +293,8 @@ __device__ __forceinline__ void for_each_exception(const MatrixDev& M, int tile,
     if (x.x == lane) f(__int_as_float(x.w), x.y, x.z);
   }
 }
+// the place words of MatrixDev::place (P4 / 4 x tiles4^2 x 16)
+void launch_places(const DevGeom& G, const MatrixDev& M, uint32_t* place, cudaStream_t st);
 // W (and, when Wh is given, the total of the half-rounded lengths) per pixel
 void launch_weights(const DevGeom& G, const MatrixDev& M, int exact, float* W,
                     float* Wh, cudaStream_t st);
@@ -256,11 +318,32 @@ TG_BACKWARD_DECL(1)
 TG_BACKWARD_DECL(2)
 TG_BACKWARD_DECL(4)
 TG_BACKWARD_DECL(8)
-TG_BACKWARD_DECL(16)
 #undef TG_BACKWARD_DECL
+void launch_backward_k16(const IterArgs& A, int batch, const float* recon_cur,
+                         float* recon_next, const float* upd, float* rep_num, int epi,
+                         cudaStream_t st);
 void launch_backward(const IterArgs& A, int batch, const float* recon_cur,
                      float* recon_next, const float* upd, float* rep_num,
                      int epi, cudaStream_t st);
+// tg_backward_mma*.cu: units first .. first + nunits - 1 of A.F (half_factors
+// != FACT_F32: halves; else floats, split: A.F.split); the multi launch serves
+// items of one (unit size, length kind, penalty, factor kind)
+void launch_backward_mma(const IterArgs& A, int first, int nunits, const float* recon_cur,
+                         float* recon_next, float* rep_num, int epi, cudaStream_t st);
+void launch_backward_mma_multi(const BackItem* items, int n, int64_t blocks, int U,
+                               int dlen_kind, int pen, int fh, cudaStream_t st);
+#define TG_MMA_DECL(KIND)                                                                  \
+  void launch_backward_mma_##KIND(const IterArgs& A, int first, int nunits,               \
+                                  const float* recon_cur, float* recon_next,              \
+                                  float* rep_num, int epi, cudaStream_t st);              \
+  void launch_backward_mma_multi_##KIND(const BackItem* items, int n, int64_t blocks,     \
+                                        int U, int pen, cudaStream_t st);
+TG_MMA_DECL(half)
+TG_MMA_DECL(split)
+TG_MMA_DECL(u16)
+TG_MMA_DECL(bf16)
+TG_MMA_DECL(f32)
+#undef TG_MMA_DECL
 // tg_backward_staged.cu (fast mode)
 void launch_backward_staged(const IterArgs& A, int batch, const float* recon_cur,
                             float* recon_next, const float* upd, float* rep_num,
@@ -320,12 +403,23 @@ void launch_runs_fill(const DevGeom& G, const MatrixDev& M, int tiles_x, int ts,
                       const int64_t* ray_run_off, const int* run_slot,
                       const int64_t* gseg_off, const int64_t* gcode_off,
                       void* tlen, uint32_t* tcode, cudaStream_t st);
-// part: [runs][K] partial sums, written (not accumulated) by each launch
+// part: [runs][K] partial sums, written (not accumulated) by each launch;
+// flag, fmax (optional): the batch's non-finite flag and its K slices'
+// largest factors, reset
 void launch_forward_tiled(const IterArgs& A, const TileMatrixDev& T,
-                          const float* recon_batch, float* part, cudaStream_t st);
+                          const float* recon_batch, float* part, int* flag, unsigned* fmax,
+                          cudaStream_t st);
 // ray sums from the partial sums (fixed order) -> per-ray values `out`
 void launch_fwd_finish(const IterArgs& A, const TileMatrixDev& T, const float* part,
                        const float* sino, float* out, int out_mode, cudaStream_t st);
+// the same, factors of slice batch `batch` into A.F
+void launch_fwd_finish_units(const IterArgs& A, const TileMatrixDev& T, const float* part,
+                             const float* sino, int batch, int out_mode, cudaStream_t st);
+// units first .. first + nunits - 1 of A.F: floats -> scaled halves (A.F.split)
+void launch_split_factors(const IterArgs& A, int first, int nunits, cudaStream_t st);
+void launch_split_factors_multi(const FinItem* items, int n, int64_t blocks, cudaStream_t st);
+// blocks of a plan's item in the multi launch
+int64_t split_blocks(const FactorDev& F, int P4, int nunits);
 // the same over many plans' slice batches in one launch each (device item
 // arrays; blocks = the launch's total blocks; all items of one launch share
 // K, the tile side and precision and the summation; 16-bit fixed-point
@@ -335,7 +429,8 @@ void launch_forward_tiled_multi(const FwdItem* items, int n, int64_t blocks, int
 void launch_fwd_finish_multi(const FinItem* items, int n, int64_t blocks, int K, int comp,
                              cudaStream_t st);
 // plans with 16-bit fixed-point lengths (backward matrix u16, or f16 with
-// half gathers); pen: PML/APMLR; fh: half factors
+// half gathers), compensated or with FP32 operands at K < 8; pen: PML/APMLR;
+// fh: half factors
 void launch_backward_multi(const BackItem* items, int n, int64_t blocks, int K,
                            int dlen_kind, int pen, int fh, int comp, cudaStream_t st);
 // blocks (of 256 threads) a plan's backprojection launch uses

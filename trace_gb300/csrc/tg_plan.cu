@@ -60,6 +60,14 @@ struct tg_plan {
   cudaEvent_t ev_dl = nullptr;
   float* d_part2 = nullptr;
   float* d_upd2 = nullptr;
+  // tensor-core backprojection: the factors of every unit of slices (F[0]:
+  // floats, F[1]: halves, allocated on first use), launched in groups of
+  // group_units; batches and streams meet at ev_meet / ev_group
+  bool mma = false;
+  FactorDev F[2] = {};
+  int unit = 0, nunits = 0, group_units = 1;  // slices per unit, units, units per group
+  int* d_flags = nullptr;
+  cudaEvent_t ev_meet = nullptr, ev_group[2] = {nullptr, nullptr};
   // FP64 mode: double state, factors, total lengths and SIRT's a2
   bool fp64 = false;
   double *d_ra2d = nullptr, *d_W64 = nullptr;
@@ -556,8 +564,34 @@ int build_tiles(tg_plan* p, int* d_nruns) {
 }
 
 int ensure_upd(tg_plan* p) {
+  if (p->mma) return TG_OK;  // ensure_factors
   if (!p->d_upd) TG_TRY(dalloc(p, &p->d_upd, (size_t)p->R * p->K * (p->fp64 ? 2 : 1)));
   if (p->two && !p->d_upd2) TG_TRY(dalloc(p, &p->d_upd2, (size_t)p->R * p->K));
+  return TG_OK;
+}
+
+// The factor units of the tensor-core backprojection (padding columns and
+// angles are zero and stay so).
+int ensure_factors(tg_plan* p, bool half) {
+  FactorDev& F = p->F[half];
+  if (!p->mma || F.base) return TG_OK;
+  FactorDev f{};
+  f.U = p->unit;
+  f.RP = factor_row(p->C);
+  f.unit_elems = (int64_t)p->M.P4 * f.RP * f.U;
+  f.ring = std::min(p->nunits, 2 * p->group_units);
+  f.blocks_x = (p->C + 15) / 16;
+  f.nflags = p->nb;
+  if (!p->d_flags) TG_TRY(dalloc(p, &p->d_flags, (size_t)p->nb, true));
+  f.flags = p->d_flags;
+  char* base = nullptr;
+  TG_TRY(dalloc(p, &base, (size_t)f.unit_elems * f.ring * (half ? 2 : 4), true));
+  f.base = base;
+  if (!half && p->M.dlen_kind == LK_F16) {
+    TG_TRY(dalloc(p, &f.split, (size_t)f.unit_elems * f.ring * 2, true));
+    TG_TRY(dalloc(p, &f.fmax, (size_t)p->nb * p->K, true));
+  }
+  F = f;
   return TG_OK;
 }
 
@@ -959,11 +993,38 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
     if (p->err.empty()) p->err = "building the tile-ordered forward matrix failed";
     return bail(rc);
   }
+  // The backprojection runs on the tensor cores for half-gather plans with
+  // 16-bit lengths (f16 in the backward matrix), and for FP32 operands at 8
+  // slices per pass. A larger unit of slices spreads a tile's A operand over
+  // more slices (1024 x 1024, 720 angles, per 8 slices: 0.96 ms in units of 8,
+  // 0.61 of 16, 0.39 of 32), but a small grid has too few blocks to fill the
+  // GPU with, so the unit is the largest one that leaves two blocks per SM.
+  // Groups of units (64 slices) are one launch.
+  p->mma = p->tiles && !d.backward_staged && !d.compensated &&
+           (d.half_gathers ? M.dlen_kind == LK_F16 : p->K == 8);
+  if (p->mma) {
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int U = p->S <= 8 ? 8 : p->S <= 16 ? 16 : 32;
+    while (U > 8 && mma_regions(C) * ((p->S + U - 1) / U) < 2 * sms) U /= 2;
+    p->unit = std::max(U, p->K);
+    p->nunits = (p->S + p->unit - 1) / p->unit;
+    p->group_units = std::min(std::max(1, 64 / p->unit), p->nunits);
+    M.tiles4 = (C + 3) / 4;
+    uint32_t* place = nullptr;
+    if ((rc = dalloc(p, &place, (size_t)M.tiles4 * M.tiles4 * 16 * (P4 / 4)))) return bail(rc);
+    launch_places(G, M, place, p->st);
+    M.place = place;
+  }
   // two-stream iterations: tile-staged plans with two or more slice batches
   if (p->tiles && p->nb >= 2 && d.batch_streams != 1) {
     if (cudaStreamCreateWithFlags(&p->st2, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&p->ev_meet, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&p->ev_group[0], cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&p->ev_group[1], cudaEventDisableTiming) != cudaSuccess) {
       cudaGetLastError();
       p->err = "creating the second stream failed";
       return bail(TG_E_CUDA);
@@ -1048,6 +1109,9 @@ int tg_plan_destroy(tg_plan* p) {
   if (p->st2) cudaStreamSynchronize(p->st2);
   if (p->ev_fork) cudaEventDestroy(p->ev_fork);
   if (p->ev_join) cudaEventDestroy(p->ev_join);
+  if (p->ev_meet) cudaEventDestroy(p->ev_meet);
+  for (auto ev : p->ev_group)
+    if (ev) cudaEventDestroy(ev);
   if (p->st2) cudaStreamDestroy(p->st2);
   if (p->st_dl) cudaStreamSynchronize(p->st_dl);
   for (auto ev : p->ev_batch) cudaEventDestroy(ev);
@@ -1199,7 +1263,7 @@ static int run_forward(tg_plan* p, const IterArgs& A0, int b, int out_mode,
     A.half_factors = 0;
     {
       Timed t(p, 0);
-      launch_forward_tiled(A, p->T, src, p->d_part, p->st);
+      launch_forward_tiled(A, p->T, src, p->d_part, nullptr, nullptr, p->st);
     }
     Timed t(p, 2);
     launch_fwd_finish(A, p->T, p->d_part,
@@ -1226,6 +1290,56 @@ static int half_factors_next(const tg_plan* p, int mode) {
   return factor_storage(p, mode, p->iters_done);
 }
 
+// The iteration of a plan with the tensor-core backprojection: every batch's
+// forward projection and finish, and per group of units one backprojection.
+// two: odd batches and odd groups run on the second stream; a group's
+// backprojection waits for the other stream's batches, and a group's finishes
+// for the backprojection that last read the units they overwrite (the ring
+// holds two groups).
+static void issue_units(tg_plan* p, IterArgs A, int mode, bool two, int epi,
+                        const std::function<void(int, cudaStream_t)>& after_batch = {}) {
+  A.F = p->F[A.half_factors != FACT_F32];
+  const float* cur = p->d_recon[p->cur];
+  const int per_group = p->group_units * A.F.U;  // slices
+  const int ngroups = (p->nunits + p->group_units - 1) / p->group_units;
+  cudaStream_t st[2] = {p->st, two ? p->st2 : p->st};
+  for (int g = 0; g < ngroups; ++g) {
+    const int b0 = g * per_group / p->K;
+    const int b1 = std::min(p->nb, (g + 1) * per_group / p->K);
+    if (two && g >= 2) cudaStreamWaitEvent(st[(g + 1) & 1], p->ev_group[g & 1], 0);
+    for (int b = b0; b < b1; ++b) {
+      const int odd = two ? b & 1 : 0;
+      float* part = odd ? p->d_part2 : p->d_part;
+      {
+        Timed t(p, 0);
+        launch_forward_tiled(A, p->T, batch_ptr(p, p->d_recon[p->cur], b * p->K + p->fshift),
+                             part, p->d_flags + b, A.F.split ? A.F.fmax + b * p->K : nullptr,
+                             st[odd]);
+      }
+      Timed t(p, 2);
+      launch_fwd_finish_units(A, p->T, part, p->d_sino + (int64_t)b * p->R * p->K, b, mode,
+                              st[odd]);
+    }
+    const cudaStream_t s = st[g & 1];
+    if (two) {
+      cudaEventRecord(p->ev_meet, st[(g + 1) & 1]);
+      cudaStreamWaitEvent(s, p->ev_meet, 0);
+    }
+    {
+      Timed t(p, 1);
+      const int first = g * p->group_units;
+      if (A.F.split)
+        launch_split_factors(A, first, std::min(p->group_units, p->nunits - first), s);
+      launch_backward_mma(A, first, std::min(p->group_units, p->nunits - first), cur,
+                          epi == EPI_UPDATE ? p->d_recon[p->cur ^ 1] : nullptr,
+                          epi == EPI_UPDATE ? nullptr : p->d_rep, epi, s);
+    }
+    if (two) cudaEventRecord(p->ev_group[g & 1], s);
+    if (after_batch)
+      for (int b = b0; b < b1; ++b) after_batch(b, s);
+  }
+}
+
 // Launches of one fused iteration on the plan's stream (buffers by p->cur;
 // the caller flips p->cur and counts the iteration).
 // two_streams: the plan's odd slice batches go to its second stream (forked
@@ -1243,7 +1357,8 @@ static void issue_iteration(tg_plan* p, const IterArgs& A0, int mode, bool two_s
     cudaEventRecord(p->ev_fork, p->st);
     cudaStreamWaitEvent(p->st2, p->ev_fork, 0);
   }
-  for (int b = 0; b < p->nb; ++b) {
+  if (p->mma) issue_units(p, A, mode, two, EPI_UPDATE, after_batch);
+  for (int b = 0; b < p->nb && !p->mma; ++b) {
     const bool odd = two && (b & 1);
     const cudaStream_t s = odd ? p->st2 : p->st;
     float* upd = odd ? p->d_upd2 : p->d_upd;
@@ -1252,7 +1367,7 @@ static void issue_iteration(tg_plan* p, const IterArgs& A0, int mode, bool two_s
       const float* src = batch_ptr(p, p->d_recon[p->cur], b * p->K + p->fshift);
       {
         Timed t(p, 0);
-        launch_forward_tiled(A, p->T, src, part, s);
+        launch_forward_tiled(A, p->T, src, part, nullptr, nullptr, s);
       }
       Timed t(p, 2);
       launch_fwd_finish(A, p->T, part, p->d_sino + (int64_t)b * p->R * p->K, upd, mode, s);
@@ -1279,6 +1394,7 @@ static int iterate_ready(tg_plan* p, int alg, const tg_params* prm) {
   TG_TRY(check_layout(p, alg));
   if (!p->have_sino) return fail(p, TG_E_STATE, "no sinogram uploaded");
   if (alg >= TG_PML && !prm) return fail(p, TG_E_ARG, "penalised algorithms need params");
+  TG_TRY(ensure_factors(p, p->d.half_gathers && alg != TG_SIRT));
   return ensure_upd(p);
 }
 
@@ -1445,7 +1561,7 @@ namespace {
 
 bool multi_eligible(const tg_plan* p) {
   return !p->fp64 && p->tiles && !p->d.backward_staged && p->d.mode == TG_MODE_FAST &&
-         p->len_kind == TG_LEN_U16;
+         p->len_kind == TG_LEN_U16 && p->nunits <= 2 * p->group_units;
 }
 
 void drop_states(tg_batch* b) {
@@ -1456,10 +1572,11 @@ void drop_states(tg_batch* b) {
   b->states.clear();
 }
 
-// A launch of the multi-plan kernels: kind 0 forward, 1 finish, 2 backward;
+// A launch of the multi-plan kernels: kind 0 forward, 1 finish, 2 backward,
+// 3 float factors to halves;
 // its items start at byte `off` of the state's item buffer.
 struct MultiLaunch {
-  int kind, branch, K, ts, bw, half_tile, comp, dlen, pen, fh;
+  int kind, branch, K, ts, bw, half_tile, comp, dlen, pen, fh, U;
   size_t off;
   int n;
   int64_t blocks;
@@ -1510,6 +1627,10 @@ void multi_build(const tg_batch* b, const int* algs, const tg_params* params, in
     const std::vector<int>& key = br.first;
     int rounds = 0;
     for (int i : br.second) rounds = std::max(rounds, b->plans[i]->nb);
+    // tensor-core backprojections: one work item per plan, after its last
+    // batch's finish
+    std::map<std::vector<int>, std::vector<BackItem>> units;
+    std::vector<FinItem> splits;  // and, before them, their factors' halves
     for (int r = 0; r < rounds; ++r) {
       std::vector<FwdItem> fwd;
       std::vector<FinItem> fin;
@@ -1523,10 +1644,13 @@ void multi_build(const tg_batch* b, const int* algs, const tg_params* params, in
         IterArgs A = make_args(p, algs[i], params ? &params[i] : nullptr);
         A.half_tile = p->d.half_gathers;
         A.half_factors = hf;
+        if (p->mma) A.F = p->F[hf != FACT_F32];
         FwdItem f{};
         f.T = p->T;
         f.recon = batch_ptr(p, p->d_recon[cur], r * p->K + p->fshift);
         f.part = p->d_part;
+        f.flag = p->mma ? p->d_flags + r : nullptr;
+        f.fmax = A.F.split ? A.F.fmax + r * p->K : nullptr;
         f.g = p->C;
         f.inv_scale = A.M.inv_scale;
         f.first = p->T.ntiles;  // block count; turned into offsets below
@@ -1542,18 +1666,36 @@ void multi_build(const tg_batch* b, const int* algs, const tg_params* params, in
         n.first = (p->R + 255) / 256;
         n.out_mode = mode;
         n.fh = hf;
+        n.F = A.F;
+        n.batch = r;
+        n.C = p->C;
         fin.push_back(n);
+        if (p->mma && r > 0) continue;
+        if (A.F.split) {
+          n.P4 = A.M.P4;
+          n.S = p->S;
+          n.nrays = (int64_t)p->nunits * A.M.P4 * A.F.RP * (A.F.U / 8);
+          n.first = split_blocks(A.F, A.M.P4, p->nunits);
+          splits.push_back(n);
+        }
         BackItem k{};
         k.A = A;
         k.batch = r;
         k.cur = p->d_recon[cur];
         k.next = p->d_recon[cur ^ 1];
         k.upd = p->d_upd;
-        k.first = backward_blocks(A);
         // both half storages share one kernel (each item carries its own)
-        back[{A.M.dlen_kind, algs[i] >= TG_PML, hf != FACT_F32}].push_back(k);
+        const std::vector<int> cls = {A.M.dlen_kind, algs[i] >= TG_PML, hf != FACT_F32, A.F.U};
+        if (p->mma) {
+          k.nunits = p->nunits;
+          k.first = mma_regions(p->C) * p->nunits;
+          units[cls].push_back(k);
+        } else {
+          k.first = backward_blocks(A);
+          back[cls].push_back(k);
+        }
       }
-      auto emit = [&](int kind, auto& items, int dlen, int pen, int fh) {
+      auto emit = [&](int kind, auto& items, int dlen, int pen, int fh, int U) {
         int64_t total = 0;
         for (auto& x : items) {
           const int64_t nb = x.first;
@@ -1571,14 +1713,17 @@ void multi_build(const tg_batch* b, const int* algs, const tg_params* params, in
         l.dlen = dlen;
         l.pen = pen;
         l.fh = fh;
+        l.U = U;
         l.off = put(items.data(), items.size() * sizeof(items[0]));
         l.n = (int)items.size();
         l.blocks = total;
         launches.push_back(l);
       };
-      emit(0, fwd, 0, 0, 0);
-      emit(1, fin, 0, 0, 0);
-      for (auto& c : back) emit(2, c.second, c.first[0], c.first[1], c.first[2]);
+      emit(0, fwd, 0, 0, 0, 0);
+      emit(1, fin, 0, 0, 0, 0);
+      if (r == rounds - 1 && !splits.empty()) emit(3, splits, 0, 0, 0, 0);
+      if (r == rounds - 1) back.merge(units);  // no class is in both: U differs
+      for (auto& c : back) emit(2, c.second, c.first[0], c.first[1], c.first[2], c.first[3]);
     }
     ++branch;
   }
@@ -1597,6 +1742,11 @@ void multi_issue(const std::vector<MultiLaunch>& launches, const char* d_items,
     else if (l.kind == 1)
       launch_fwd_finish_multi(static_cast<const FinItem*>(items), l.n, l.blocks, l.K, l.comp,
                               st);
+    else if (l.kind == 3)
+      launch_split_factors_multi(static_cast<const FinItem*>(items), l.n, l.blocks, st);
+    else if (l.U)
+      launch_backward_mma_multi(static_cast<const BackItem*>(items), l.n, l.blocks, l.U, l.dlen,
+                                l.pen, l.fh, st);
     else
       launch_backward_multi(static_cast<const BackItem*>(items), l.n, l.blocks, l.K, l.dlen,
                             l.pen, l.fh, l.comp, st);
@@ -1772,7 +1922,16 @@ extern "C" int tg_batch_iterate(tg_batch* b, const int* algs, const tg_params* p
     return TG_OK;
   }
   b->last_launches = 0;
-  for (tg_plan* p : b->plans) b->last_launches += p->nb * (p->tiles ? 3 : 2);
+  for (int i = 0; i < n; ++i) {
+    const tg_plan* p = b->plans[i];
+    // tensor-core backprojection: one launch per group of units, two where
+    // float factors are split
+    const int mode = algs[i] == TG_SIRT ? FWD_SIRT : FWD_RATIO;
+    const bool split = p->F[half_factors_next(p, mode) != FACT_F32].split != nullptr;
+    b->last_launches += p->mma ? p->nb * 2 + (p->nunits + p->group_units - 1) / p->group_units *
+                                                (split ? 2 : 1)
+                               : p->nb * (p->tiles ? 3 : 2);
+  }
   for (int it = 0; it < n_iter; ++it) {
     const int parity = b->plans[0]->cur;
     tg_batch::Graph& g = b->graphs[parity];
@@ -1844,11 +2003,16 @@ int tg_reduce(tg_plan* p, int alg, const tg_params* prm) {
   TG_TRY(fp32_only(p));
   TG_TRY(check_layout(p, alg));
   if (!p->have_sino) return fail(p, TG_E_STATE, "no sinogram uploaded");
+  TG_TRY(ensure_factors(p, false));
   TG_TRY(ensure_upd(p));
   if (!p->d_rep) TG_TRY(dalloc(p, &p->d_rep, (size_t)p->S * p->g2, true));
-  const IterArgs A = make_args(p, alg, prm);
+  IterArgs A = make_args(p, alg, prm);
   const int mode = alg == TG_SIRT ? FWD_SIRT : FWD_RATIO;
-  for (int b = 0; b < p->nb; ++b) {
+  if (p->mma) {
+    A.half_tile = p->d.half_gathers;
+    issue_units(p, A, mode, false, EPI_REPLICA);
+  }
+  for (int b = 0; b < p->nb && !p->mma; ++b) {
     run_forward(p, A, b, mode, p->d_upd);
     Timed t(p, 1);
     if (!p->d.backward_staged)

@@ -491,8 +491,12 @@ template <int K, int LK, bool H, bool COMP>
 __device__ __forceinline__ void forward_tiled_block(const TileMatrixDev& T, int g,
                                                     float inv_scale, int splits, int block,
                                                     const float* __restrict__ recon,
-                                                    float* __restrict__ part) {
+                                                    float* __restrict__ part, int* flag, unsigned* fmax) {
   extern __shared__ float4 smem4[];
+  if (block == 0 && threadIdx.x < K) {
+    if (flag && threadIdx.x == 0) *flag = 0;
+    if (fmax) fmax[threadIdx.x] = 0u;
+  }
   float* sm = reinterpret_cast<float*>(smem4);
   __half* smh = reinterpret_cast<__half*>(smem4);
   // `splits` blocks share a tile (small grids: fewer tiles than SMs); each
@@ -566,8 +570,9 @@ __device__ __forceinline__ void forward_tiled_block(const TileMatrixDev& T, int 
 template <int K, int LK, bool H, bool COMP>
 __global__ void __launch_bounds__(kBlock)
     k_forward_tiled(TileMatrixDev T, int g, float inv_scale, int splits,
-                    const float* __restrict__ recon, float* __restrict__ part) {
-  forward_tiled_block<K, LK, H, COMP>(T, g, inv_scale, splits, blockIdx.x, recon, part);
+                    const float* __restrict__ recon, float* __restrict__ part, int* flag,
+                    unsigned* fmax) {
+  forward_tiled_block<K, LK, H, COMP>(T, g, inv_scale, splits, blockIdx.x, recon, part, flag, fmax);
 }
 
 // Many plans' forward projections in one launch: block -> work item (a
@@ -577,25 +582,17 @@ __global__ void __launch_bounds__(kBlock)
     k_forward_tiled_multi(const FwdItem* __restrict__ items, int nitems) {
   const FwdItem& it = items[item_of(items, nitems, blockIdx.x)];
   forward_tiled_block<K, LK, H, COMP>(it.T, it.g, it.inv_scale, 1,
-                                      (int)(blockIdx.x - it.first), it.recon, it.part);
+                                      (int)(blockIdx.x - it.first), it.recon, it.part, it.flag, it.fmax);
 }
 
-// A ray's partial sums (its runs' slots, in path order) -> per-ray factor,
-// as k_forward's epilogue. FH (ratio factors only): the factor is stored as
-// the half (ray/sim - fofs), fofs = factor_offset(storage).
-template <int K, bool FH, bool COMP>
-__device__ __forceinline__ void fwd_finish_ray(int64_t r, const int* __restrict__ rnrun,
-                                               const int* __restrict__ pbase,
-                                               const float* __restrict__ ra2,
-                                               const float* __restrict__ part,
-                                               const float* __restrict__ sino,
-                                               float* __restrict__ out, int out_mode,
-                                               float fofs) {
+// A ray's sums: its partial sums (its runs' slots) added in path order.
+template <int K, bool COMP>
+__device__ __forceinline__ Vec<K> ray_sums(int64_t r, int n, const int* __restrict__ pbase,
+                                           const float* __restrict__ part) {
   Vec<K> s;
   float cmp[K];
 #pragma unroll
   for (int j = 0; j < K; ++j) s.v[j] = cmp[j] = 0.f;
-  const int n = rnrun[r];
   // the warp's 32 rays are one ray group: run k of every lane is one row
   const float* src = part + ((int64_t)pbase[r >> 5] + (r & 31)) * K;
   for (int k = 0; k < n; ++k) {
@@ -610,17 +607,36 @@ __device__ __forceinline__ void fwd_finish_ray(int64_t r, const int* __restrict_
 #pragma unroll
     for (int j = 0; j < K; ++j) s.v[j] = fsub(s.v[j], cmp[j]);
   }
+  return s;
+}
+
+// Ray sums -> per-ray values, as k_forward's epilogue.
+template <int K>
+__device__ __forceinline__ Vec<K> ray_values(int64_t r, const Vec<K>& s,
+                                             const float* __restrict__ ra2,
+                                             const float* __restrict__ sino, int out_mode) {
+  if (out_mode == FWD_SIM) return s;
   Vec<K> o;
-  if (out_mode == FWD_SIM) {
-    o = s;
-  } else {
-    const Vec<K> ray = load_vec<K>(sino + r * K);
-    const float a2 = out_mode == FWD_SIRT ? ra2[r] : 1.f;
+  const Vec<K> ray = load_vec<K>(sino + r * K);
+  const float a2 = out_mode == FWD_SIRT ? ra2[r] : 1.f;
 #pragma unroll
-    for (int j = 0; j < K; ++j)
-      o.v[j] = out_mode == FWD_SIRT ? fdiv(fsub(ray.v[j], s.v[j]), a2)
-                                    : fdiv(ray.v[j], s.v[j]);
-  }
+  for (int j = 0; j < K; ++j)
+    o.v[j] = out_mode == FWD_SIRT ? fdiv(fsub(ray.v[j], s.v[j]), a2)
+                                  : fdiv(ray.v[j], s.v[j]);
+  return o;
+}
+
+// FH (ratio factors only): the factor is stored as the half
+// (ray/sim - fofs), fofs = factor_offset(storage).
+template <int K, bool FH, bool COMP>
+__device__ __forceinline__ void fwd_finish_ray(int64_t r, const int* __restrict__ rnrun,
+                                               const int* __restrict__ pbase,
+                                               const float* __restrict__ ra2,
+                                               const float* __restrict__ part,
+                                               const float* __restrict__ sino,
+                                               float* __restrict__ out, int out_mode,
+                                               float fofs) {
+  Vec<K> o = ray_values<K>(r, ray_sums<K, COMP>(r, rnrun[r], pbase, part), ra2, sino, out_mode);
   if constexpr (FH) {
 #pragma unroll
     for (int j = 0; j < K; ++j) o.v[j] -= fofs;
@@ -628,6 +644,103 @@ __device__ __forceinline__ void fwd_finish_ray(int64_t r, const int* __restrict_
   } else {
     store_vec<K>(out + r * K, o);
   }
+}
+
+// The same into the units of the tensor-core backprojection (FactorDev).
+// Rays without segments store 0 (no pixel uses them); a non-finite factor
+// raises the batch's flag.
+template <int K, bool FH>
+__device__ __forceinline__ void finish_units_ray(int64_t r, const FactorDev& F, int C, int batch,
+                                                 const int* __restrict__ rnrun,
+                                                 const int* __restrict__ pbase,
+                                                 const float* __restrict__ ra2,
+                                                 const float* __restrict__ part,
+                                                 const float* __restrict__ sino, int out_mode,
+                                                 float fofs) {
+  Vec<K> o;
+#pragma unroll
+  for (int j = 0; j < K; ++j) o.v[j] = 0.f;
+  const int n = rnrun[r];
+  if (n > 0) {
+    o = ray_values<K>(r, ray_sums<K, false>(r, n, pbase, part), ra2, sino, out_mode);
+    if constexpr (FH) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) o.v[j] -= fofs;
+    }
+  }
+  const int a = (int)(r / C), c = (int)(r - (int64_t)a * C);
+  const int unit = batch * K / F.U, su = batch * K % F.U;
+  const int64_t e = factor_at((int64_t)(unit % F.ring) * F.unit_elems, F.RP, F.U, a, c, su);
+  bool bad = false;
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    // halves: what rounds to infinity too; floats: the top of the range too,
+    // where rounding up to the TF32 part may overflow
+    if constexpr (FH) bad |= !(fabsf(__half2float(__float2half_rn(o.v[j]))) < 7e4f);
+    else bad |= !(fabsf(o.v[j]) < 1e38f);
+  }
+  if constexpr (FH) {
+    store_hvec<K>(reinterpret_cast<__half*>(F.base) + e, o);
+  } else {
+    store_vec<K>(reinterpret_cast<float*>(F.base) + e, o);
+    if (F.split) {  // the slices' largest factors (the order of their bits)
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        const unsigned act = __activemask();
+        const unsigned m = __reduce_max_sync(act, __float_as_uint(fabsf(o.v[j])));
+        if ((threadIdx.x & 31) == __ffs(act) - 1 && m > F.fmax[batch * K + j])
+          atomicMax(F.fmax + batch * K + j, m);
+      }
+    }
+  }
+  if (bad) F.flags[batch] = 1;
+}
+
+// Float factors of one column and 8 slices -> high and low halves (FactorDev).
+// `i` counts (unit from `first`, angle, column, 8 slices).
+__device__ __forceinline__ void split_factors(const FactorDev& F, int P4, int S, int first,
+                                              int64_t i) {
+  const int oct = F.U / 8;
+  const int o = (int)(i % oct);
+  const int64_t col = i / oct;  // unit, angle and column
+  const int64_t per_unit = (int64_t)P4 * F.RP;
+  const int unit = first + (int)(col / per_unit);
+  const int64_t e = (int64_t)(unit % F.ring) * F.unit_elems + col % per_unit * F.U + o * 8;
+  const Vec<8> v = load_vec<8>(reinterpret_cast<const float*>(F.base) + e);
+  Vec<8> hi, lo;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int s = unit * F.U + o * 8 + j;
+    const float x = v.v[j] * (s < S ? split_scale(F.fmax[s]) : 1.f);
+    hi.v[j] = __half2float(__float2half_rn(x));
+    lo.v[j] = fsub(x, hi.v[j]);
+  }
+  __half* dst = F.split + (e - o * 8) * 2 + o * 8;
+  store_hvec<8>(dst, hi);
+  store_hvec<8>(dst + F.U, lo);
+}
+
+__global__ void k_split_factors(const __grid_constant__ FactorDev F, int P4, int S, int first,
+                                int64_t n) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) split_factors(F, P4, S, first, i);
+}
+
+__global__ void k_split_factors_multi(const FinItem* __restrict__ items, int nitems) {
+  const FinItem& it = items[item_of(items, nitems, blockIdx.x)];
+  const int64_t i = (int64_t)(blockIdx.x - it.first) * blockDim.x + threadIdx.x;
+  if (i < it.nrays) split_factors(it.F, it.P4, it.S, 0, i);
+}
+
+template <int K, bool FH>
+__global__ void k_fwd_finish_units(int64_t nrays, const __grid_constant__ FactorDev F, int C,
+                                   int batch, const int* __restrict__ rnrun,
+                                   const int* __restrict__ pbase, const float* __restrict__ ra2,
+                                   const float* __restrict__ part,
+                                   const float* __restrict__ sino, int out_mode, float fofs) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < nrays)
+    finish_units_ray<K, FH>(r, F, C, batch, rnrun, pbase, ra2, part, sino, out_mode, fofs);
 }
 
 template <int K, bool FH, bool COMP>
@@ -648,6 +761,15 @@ __global__ void k_fwd_finish_multi(const FinItem* __restrict__ items, int nitems
   const FinItem& it = items[item_of(items, nitems, blockIdx.x)];
   const int64_t r = (int64_t)(blockIdx.x - it.first) * blockDim.x + threadIdx.x;
   if (r >= it.nrays) return;
+  if (!COMP && it.F.U) {
+    if (it.fh != FACT_F32)
+      finish_units_ray<K, true>(r, it.F, it.C, it.batch, it.rnrun, it.pbase, it.ra2,
+                                it.part, it.sino, it.out_mode, factor_offset(it.fh));
+    else
+      finish_units_ray<K, false>(r, it.F, it.C, it.batch, it.rnrun, it.pbase, it.ra2,
+                                 it.part, it.sino, it.out_mode, 0.f);
+    return;
+  }
   if (it.fh != FACT_F32)
     fwd_finish_ray<K, true, COMP>(r, it.rnrun, it.pbase, it.ra2, it.part, it.sino, it.out,
                                   it.out_mode, factor_offset(it.fh));
@@ -658,7 +780,7 @@ __global__ void k_fwd_finish_multi(const FinItem* __restrict__ items, int nitems
 
 template <int K, int LK, bool H, bool COMP>
 void fwd_tiled_launch(const TileMatrixDev& T, int g, float inv_scale,
-                      const float* recon, float* part, cudaStream_t st) {
+                      const float* recon, float* part, int* flag, unsigned* fmax, cudaStream_t st) {
   const int smem = TilePlanes<K, H>::bytes(T.ts);
   cudaFuncSetAttribute(k_forward_tiled<K, LK, H, COMP>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -668,38 +790,38 @@ void fwd_tiled_launch(const TileMatrixDev& T, int g, float inv_scale,
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int splits = max(1, min(16, (2 * sms + T.ntiles - 1) / T.ntiles));
   k_forward_tiled<K, LK, H, COMP><<<T.ntiles * splits, T.bw * 32, smem, st>>>(
-      T, g, inv_scale, splits, recon, part);
+      T, g, inv_scale, splits, recon, part, flag, fmax);
 }
 
 template <int K, bool H, bool COMP>
 void fwd_tiled_kind(const TileMatrixDev& T, int g, int len_kind, float inv_scale,
-                    const float* recon, float* part, cudaStream_t st) {
+                    const float* recon, float* part, int* flag, unsigned* fmax, cudaStream_t st) {
   switch (len_kind) {
-    case LK_F32: fwd_tiled_launch<K, LK_F32, H, COMP>(T, g, inv_scale, recon, part, st); break;
-    case LK_BF16: fwd_tiled_launch<K, LK_BF16, H, COMP>(T, g, inv_scale, recon, part, st); break;
-    case LK_F16: fwd_tiled_launch<K, LK_F16, H, COMP>(T, g, inv_scale, recon, part, st); break;
-    default: fwd_tiled_launch<K, LK_U16, H, COMP>(T, g, inv_scale, recon, part, st); break;
+    case LK_F32: fwd_tiled_launch<K, LK_F32, H, COMP>(T, g, inv_scale, recon, part, flag, fmax, st); break;
+    case LK_BF16: fwd_tiled_launch<K, LK_BF16, H, COMP>(T, g, inv_scale, recon, part, flag, fmax, st); break;
+    case LK_F16: fwd_tiled_launch<K, LK_F16, H, COMP>(T, g, inv_scale, recon, part, flag, fmax, st); break;
+    default: fwd_tiled_launch<K, LK_U16, H, COMP>(T, g, inv_scale, recon, part, flag, fmax, st); break;
   }
 }
 
 template <int K, bool COMP>
 void fwd_tiled_half(const IterArgs& A, const TileMatrixDev& T, const float* recon,
-                    float* part, cudaStream_t st) {
+                    float* part, int* flag, unsigned* fmax, cudaStream_t st) {
   // an f32 tile of 16 slices would not fit shared memory (plan creation
   // requires half_gathers with 16 slices per pass and forward_tiles)
   if (K == 16 || A.half_tile)
-    fwd_tiled_kind<K, true, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, st);
+    fwd_tiled_kind<K, true, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, flag, fmax, st);
   else if constexpr (K != 16)
-    fwd_tiled_kind<K, false, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, st);
+    fwd_tiled_kind<K, false, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, flag, fmax, st);
 }
 
 // compensated sums: up to 8 slices per pass (plan creation checks)
 template <int K>
 void fwd_tiled_comp(const IterArgs& A, const TileMatrixDev& T, const float* recon,
-                    float* part, cudaStream_t st) {
+                    float* part, int* flag, unsigned* fmax, cudaStream_t st) {
   constexpr bool kComp = K <= 8;
-  if (kComp && A.comp) fwd_tiled_half<K, kComp>(A, T, recon, part, st);
-  else fwd_tiled_half<K, false>(A, T, recon, part, st);
+  if (kComp && A.comp) fwd_tiled_half<K, kComp>(A, T, recon, part, flag, fmax, st);
+  else fwd_tiled_half<K, false>(A, T, recon, part, flag, fmax, st);
 }
 
 inline int blocks_for(int64_t n, int b) { return (int)((n + b - 1) / b); }
@@ -832,13 +954,13 @@ void launch_runs_fill(const DevGeom& G, const MatrixDev& M, int tiles_x, int ts,
 }
 
 void launch_forward_tiled(const IterArgs& A, const TileMatrixDev& T,
-                          const float* recon_batch, float* part, cudaStream_t st) {
+                          const float* recon_batch, float* part, int* flag, unsigned* fmax, cudaStream_t st) {
   switch (A.K) {
-    case 1: fwd_tiled_comp<1>(A, T, recon_batch, part, st); break;
-    case 2: fwd_tiled_comp<2>(A, T, recon_batch, part, st); break;
-    case 4: fwd_tiled_comp<4>(A, T, recon_batch, part, st); break;
-    case 8: fwd_tiled_comp<8>(A, T, recon_batch, part, st); break;
-    default: fwd_tiled_comp<16>(A, T, recon_batch, part, st); break;
+    case 1: fwd_tiled_comp<1>(A, T, recon_batch, part, flag, fmax, st); break;
+    case 2: fwd_tiled_comp<2>(A, T, recon_batch, part, flag, fmax, st); break;
+    case 4: fwd_tiled_comp<4>(A, T, recon_batch, part, flag, fmax, st); break;
+    case 8: fwd_tiled_comp<8>(A, T, recon_batch, part, flag, fmax, st); break;
+    default: fwd_tiled_comp<16>(A, T, recon_batch, part, flag, fmax, st); break;
   }
 }
 
@@ -869,6 +991,45 @@ void launch_fwd_finish(const IterArgs& A, const TileMatrixDev& T, const float* p
     case 8: fwd_finish_k<8>(A, T, part, sino, out, out_mode, st); break;
     default: fwd_finish_k<16>(A, T, part, sino, out, out_mode, st); break;
   }
+}
+
+template <int K>
+static void finish_units_k(const IterArgs& A, const TileMatrixDev& T, const float* part,
+                           const float* sino, int batch, int out_mode, cudaStream_t st) {
+  const int64_t R = (int64_t)A.G.P * A.G.C;
+  const int b = blocks_for(R, 256);
+  if (A.half_factors != FACT_F32)
+    k_fwd_finish_units<K, true><<<b, 256, 0, st>>>(R, A.F, A.G.C, batch, T.rnrun, T.pbase,
+                                                   A.M.ra2, part, sino, out_mode,
+                                                   factor_offset(A.half_factors));
+  else
+    k_fwd_finish_units<K, false><<<b, 256, 0, st>>>(R, A.F, A.G.C, batch, T.rnrun, T.pbase,
+                                                    A.M.ra2, part, sino, out_mode, 0.f);
+}
+
+void launch_fwd_finish_units(const IterArgs& A, const TileMatrixDev& T, const float* part,
+                             const float* sino, int batch, int out_mode, cudaStream_t st) {
+  switch (A.K) {
+    case 1: finish_units_k<1>(A, T, part, sino, batch, out_mode, st); break;
+    case 2: finish_units_k<2>(A, T, part, sino, batch, out_mode, st); break;
+    case 4: finish_units_k<4>(A, T, part, sino, batch, out_mode, st); break;
+    case 8: finish_units_k<8>(A, T, part, sino, batch, out_mode, st); break;
+    default: finish_units_k<16>(A, T, part, sino, batch, out_mode, st); break;
+  }
+}
+
+static int64_t split_count(const FactorDev& F, int P4, int nunits) {
+  return (int64_t)nunits * P4 * F.RP * (F.U / 8);
+}
+int64_t split_blocks(const FactorDev& F, int P4, int nunits) {
+  return (split_count(F, P4, nunits) + 255) / 256;
+}
+void launch_split_factors(const IterArgs& A, int first, int nunits, cudaStream_t st) {
+  const int64_t n = split_count(A.F, A.M.P4, nunits);
+  k_split_factors<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A.F, A.M.P4, A.S, first, n);
+}
+void launch_split_factors_multi(const FinItem* items, int n, int64_t blocks, cudaStream_t st) {
+  k_split_factors_multi<<<(unsigned)blocks, 256, 0, st>>>(items, n);
 }
 
 template <int K, int LK, bool H, bool COMP>

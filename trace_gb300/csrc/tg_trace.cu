@@ -219,6 +219,35 @@ __global__ void k_weights(DevGeom G, MatrixDev M, int exact, float* W, float* Wh
   if constexpr (HALF) Wh[p] = sumh;
 }
 
+// What the tensor-core backprojection needs of the pixel's place o = 0..6 in
+// its tile's window of eight columns, as one byte: 8 o (a byte shift; bit 5 is
+// the place of its part in the upper group of halves), bit 6 that in the lower
+// group ((o + 1) / 4), bit 7 that in the even group of floats ((o + 1) / 2,
+// odd part; the odd group's is bit 4).
+__device__ __forceinline__ uint32_t place_byte(int o) {
+  return (uint32_t)(8 * o) | (uint32_t)(((o + 1) >> 2) << 6) |
+         (uint32_t)((((o + 1) >> 1) & 1) << 7);
+}
+
+__global__ void k_places(DevGeom G, MatrixDev M, uint32_t* place) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t per_quad = (int64_t)M.tiles4 * M.tiles4 * 16;
+  if (i >= per_quad * (M.P4 / 4)) return;
+  const int quad = (int)(i / per_quad);
+  const int64_t k = i - (int64_t)quad * per_quad;
+  const int tile = (int)(k >> 4), w = (int)k & 15;
+  const int px = (w >> 1) | ((w & 1) << 3);
+  const int tx = tile % M.tiles4 * 4, ty = tile / M.tiles4 * 4;
+  const float xf = (float)(tx + (px & 3)), yf = (float)(ty + (px >> 2));
+  uint32_t word = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float4 cf = M.wcoef[quad * 4 + j];
+    word |= place_byte(window_bits(cf, xf, yf) - window_low(cf, tx, ty, 4, 4)) << (8 * j);
+  }
+  place[i] = word;
+}
+
 __global__ void __launch_bounds__(kTraceBlock)
     k_trace_export(DevGeom G, int nrays, const int64_t* offsets, int* idx,
                    float* len, float* len2) {
@@ -285,6 +314,11 @@ void launch_weights(const DevGeom& G, const MatrixDev& M, int exact, float* W,
     else
       k_weights<false, false><<<blocks, 256, 0, st>>>(G, M, exact, W, Wh);
   }
+}
+
+void launch_places(const DevGeom& G, const MatrixDev& M, uint32_t* place, cudaStream_t st) {
+  const int64_t n = (int64_t)M.tiles4 * M.tiles4 * 16 * (M.P4 / 4);
+  k_places<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(G, M, place);
 }
 
 void launch_trace_export(const DevGeom& G, const int64_t* offsets, int* idx,
