@@ -22,15 +22,15 @@ void launch_backward_multi(const BackItem* items, int n, int64_t blocks, int K,
 
 int64_t backward_blocks(const IterArgs& A) { return (A.M.ntiles + kWarps - 1) / kWarps; }
 
-void launch_backward(const IterArgs& A, int batch, const float* recon_cur,
+void launch_backward(const IterArgs& A, int first, int nb, const float* recon_cur,
                      float* recon_next, const float* upd, float* rep_num,
                      int epi, cudaStream_t st) {
   switch (A.K) {
-    case 1: launch_backward_k1(A, batch, recon_cur, recon_next, upd, rep_num, epi, st); break;
-    case 2: launch_backward_k2(A, batch, recon_cur, recon_next, upd, rep_num, epi, st); break;
-    case 4: launch_backward_k4(A, batch, recon_cur, recon_next, upd, rep_num, epi, st); break;
-    case 8: launch_backward_k8(A, batch, recon_cur, recon_next, upd, rep_num, epi, st); break;
-    default: launch_backward_k16(A, batch, recon_cur, recon_next, upd, rep_num, epi, st); break;
+    case 1: launch_backward_k1(A, first, nb, recon_cur, recon_next, upd, rep_num, epi, st); break;
+    case 2: launch_backward_k2(A, first, nb, recon_cur, recon_next, upd, rep_num, epi, st); break;
+    case 4: launch_backward_k4(A, first, nb, recon_cur, recon_next, upd, rep_num, epi, st); break;
+    case 8: launch_backward_k8(A, first, nb, recon_cur, recon_next, upd, rep_num, epi, st); break;
+    default: launch_backward_k16(A, first, nb, recon_cur, recon_next, upd, rep_num, epi, st); break;
   }
 }
 

@@ -371,12 +371,19 @@ __device__ __forceinline__ void backward_block(const IterArgs& A, int batch, int
 
 template <int K, int LK, bool EXACT, bool PEN, bool FH, bool COMP>
 __global__ void __launch_bounds__(kBlock, (min_blocks<K, COMP>()))
-    k_backward(IterArgs A, int batch, const float* __restrict__ cur,
+    k_backward(IterArgs A, int first, int nb, const float* __restrict__ cur,
                float* __restrict__ next, const float* __restrict__ upd,
                float* __restrict__ rep_num, int epi) {
   __shared__ float4 s_coef[kCoefChunk];
-  backward_block<K, LK, EXACT, PEN, FH, COMP>(A, batch, blockIdx.x, cur, next, upd,
-                                              rep_num, epi, s_coef);
+  // batches first .. first + nb - 1, each with its factors behind the other:
+  // consecutive blocks take the same pixels of all of them, so that they read
+  // a piece of the matrix while it is in L2
+  const int blk = blockIdx.x / nb, b = blockIdx.x - blk * nb;
+  const float* u = FH ? reinterpret_cast<const float*>(
+                            reinterpret_cast<const __half*>(upd) + b * ((int64_t)A.G.P * A.G.C * K))
+                      : upd + b * ((int64_t)A.G.P * A.G.C * K);
+  backward_block<K, LK, EXACT, PEN, FH, COMP>(A, first + b, blk, cur, next, u, rep_num, epi,
+                                              s_coef);
 }
 
 // Many plans' fused backprojection + update in one launch (fast mode):
@@ -415,13 +422,13 @@ void back_multi(const BackItem* items, int n, int64_t blocks, int dlen_kind, int
 }
 
 template <int K, int LK>
-void back_launch(const IterArgs& A, int batch, const float* cur, float* next,
+void back_launch(const IterArgs& A, int first, int nb, const float* cur, float* next,
                  const float* upd, float* rep_num, int epi, cudaStream_t st) {
-  const int blocks = (A.M.ntiles + kWarps - 1) / kWarps;
+  const int blocks = (A.M.ntiles + kWarps - 1) / kWarps * nb;
   const bool pen = A.alg >= 2;
 #define TG_BACK(E, PN, FH, CP)                                                        \
-  k_backward<K, LK, E, PN, FH, CP><<<blocks, kBlock, 0, st>>>(A, batch, cur, next, upd, \
-                                                             rep_num, epi)
+  k_backward<K, LK, E, PN, FH, CP><<<blocks, kBlock, 0, st>>>(A, first, nb, cur, next, \
+                                                             upd, rep_num, epi)
   // compensated sums: up to 8 slices per pass (plan creation checks)
   constexpr bool kComp = K <= 8;
   if (A.exact) {
@@ -445,13 +452,13 @@ void back_launch(const IterArgs& A, int batch, const float* cur, float* next,
 }
 
 template <int K>
-void back_kind(const IterArgs& A, int batch, const float* cur, float* next,
+void back_kind(const IterArgs& A, int first, int nb, const float* cur, float* next,
                const float* upd, float* rep_num, int epi, cudaStream_t st) {
   switch (A.M.dlen_kind) {
-    case LK_F32: back_launch<K, LK_F32>(A, batch, cur, next, upd, rep_num, epi, st); break;
-    case LK_BF16: back_launch<K, LK_BF16>(A, batch, cur, next, upd, rep_num, epi, st); break;
-    case LK_F16: back_launch<K, LK_F16>(A, batch, cur, next, upd, rep_num, epi, st); break;
-    default: back_launch<K, LK_U16>(A, batch, cur, next, upd, rep_num, epi, st); break;
+    case LK_F32: back_launch<K, LK_F32>(A, first, nb, cur, next, upd, rep_num, epi, st); break;
+    case LK_BF16: back_launch<K, LK_BF16>(A, first, nb, cur, next, upd, rep_num, epi, st); break;
+    case LK_F16: back_launch<K, LK_F16>(A, first, nb, cur, next, upd, rep_num, epi, st); break;
+    default: back_launch<K, LK_U16>(A, first, nb, cur, next, upd, rep_num, epi, st); break;
   }
 }
 
@@ -461,10 +468,11 @@ void back_kind(const IterArgs& A, int batch, const float* cur, float* next,
 // unit (tg_backward*.cu) so the template instances build in parallel; the
 // multi-plan launches serve up to 8 slices per pass.
 #define TG_BACKWARD_ENTRY(KK)                                                           \
-  void launch_backward_k##KK(const IterArgs& A, int batch, const float* recon_cur,     \
-                             float* recon_next, const float* upd, float* rep_num,      \
-                             int epi, cudaStream_t st) {                               \
-    back_kind<KK>(A, batch, recon_cur, recon_next, upd, rep_num, epi, st);             \
+  void launch_backward_k##KK(const IterArgs& A, int first, int nb,                     \
+                             const float* recon_cur, float* recon_next,                \
+                             const float* upd, float* rep_num, int epi,                \
+                             cudaStream_t st) {                                        \
+    back_kind<KK>(A, first, nb, recon_cur, recon_next, upd, rep_num, epi, st);         \
   }
 #define TG_BACKWARD_MULTI_ENTRY(KK)                                                     \
   void launch_backward_multi_k##KK(const BackItem* items, int n, int64_t blocks,       \

@@ -53,12 +53,28 @@ __device__ __forceinline__ void fwd_epilogue(const MatrixDev& M, int64_t r,
   store_vec<K>(out + r * K, o);
 }
 
+// Slice batches of one launch: consecutive blocks take the same rays of the nb
+// batches, so that all of them read a piece of the matrix while it is in L2.
+// Moves the pointers to the block's batch; returns its place in the rays.
+template <int K>
+__device__ __forceinline__ int batch_block(const DevGeom& G, int nb,
+                                           const float* __restrict__& recon,
+                                           const float* __restrict__& sino,
+                                           float* __restrict__& out) {
+  const int blk = blockIdx.x / nb, b = blockIdx.x - blk * nb;
+  const int64_t rays = (int64_t)G.P * G.C * K;
+  recon += b * ((int64_t)G.C * G.C * K);
+  sino += b * rays;
+  out += b * rays;
+  return blk;
+}
+
 template <int K, int LK, bool EXACT, bool DELTA>
 __global__ void __launch_bounds__(kBlock)
-    k_forward(DevGeom G, MatrixDev M, int ngroups,
+    k_forward(DevGeom G, MatrixDev M, int ngroups, int nb,
               const float* __restrict__ recon, const float* __restrict__ sino,
               float* __restrict__ out, int out_mode) {
-  const int grp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int grp = (batch_block<K>(G, nb, recon, sino, out) * kBlock + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (grp >= ngroups) return;  // warp-uniform
   const int a = grp / G.gpa;
@@ -114,10 +130,10 @@ __global__ void __launch_bounds__(kBlock)
 // the cost moves from streaming the matrix to tracing (ALU).
 template <int K, bool EXACT>
 __global__ void __launch_bounds__(kBlock)
-    k_forward_otf(DevGeom G, MatrixDev M, int ngroups,
+    k_forward_otf(DevGeom G, MatrixDev M, int ngroups, int nb,
                   const float* __restrict__ recon, const float* __restrict__ sino,
                   float* __restrict__ out, int out_mode) {
-  const int grp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int grp = (batch_block<K>(G, nb, recon, sino, out) * kBlock + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (grp >= ngroups) return;
   const int a = grp / G.gpa;
@@ -140,12 +156,12 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 template <int K, int LK>
-void fwd_launch(const IterArgs& A, const float* recon, const float* sino,
+void fwd_launch(const IterArgs& A, int nb, const float* recon, const float* sino,
                 float* out, int out_mode, cudaStream_t st) {
   const int ngroups = A.G.P * A.G.gpa;
-  const int blocks = (int)(((int64_t)ngroups * 32 + kBlock - 1) / kBlock);
+  const int blocks = (int)(((int64_t)ngroups * 32 + kBlock - 1) / kBlock) * nb;
 #define TG_FWD(E, D) \
-  k_forward<K, LK, E, D><<<blocks, kBlock, 0, st>>>(A.G, A.M, ngroups, recon, sino, out, out_mode)
+  k_forward<K, LK, E, D><<<blocks, kBlock, 0, st>>>(A.G, A.M, ngroups, nb, recon, sino, out, out_mode)
   if (A.delta_index) {
     if (A.exact) TG_FWD(true, true); else TG_FWD(false, true);
   } else {
@@ -155,38 +171,38 @@ void fwd_launch(const IterArgs& A, const float* recon, const float* sino,
 }
 
 template <int K>
-void fwd_kind(const IterArgs& A, const float* recon, const float* sino,
+void fwd_kind(const IterArgs& A, int nb, const float* recon, const float* sino,
               float* out, int out_mode, cudaStream_t st) {
   if (A.M.rlen == nullptr) {  // no stored forward matrix: trace on the fly
     const int ngroups = A.G.P * A.G.gpa;
-    const int blocks = (int)(((int64_t)ngroups * 32 + kBlock - 1) / kBlock);
+    const int blocks = (int)(((int64_t)ngroups * 32 + kBlock - 1) / kBlock) * nb;
     if (A.exact)
-      k_forward_otf<K, true><<<blocks, kBlock, 0, st>>>(A.G, A.M, ngroups, recon, sino,
+      k_forward_otf<K, true><<<blocks, kBlock, 0, st>>>(A.G, A.M, ngroups, nb, recon, sino,
                                                          out, out_mode);
     else
-      k_forward_otf<K, false><<<blocks, kBlock, 0, st>>>(A.G, A.M, ngroups, recon, sino,
+      k_forward_otf<K, false><<<blocks, kBlock, 0, st>>>(A.G, A.M, ngroups, nb, recon, sino,
                                                           out, out_mode);
     return;
   }
   switch (A.M.len_kind) {
-    case LK_F32: fwd_launch<K, LK_F32>(A, recon, sino, out, out_mode, st); break;
-    case LK_BF16: fwd_launch<K, LK_BF16>(A, recon, sino, out, out_mode, st); break;
-    case LK_F16: fwd_launch<K, LK_F16>(A, recon, sino, out, out_mode, st); break;
-    default: fwd_launch<K, LK_U16>(A, recon, sino, out, out_mode, st); break;
+    case LK_F32: fwd_launch<K, LK_F32>(A, nb, recon, sino, out, out_mode, st); break;
+    case LK_BF16: fwd_launch<K, LK_BF16>(A, nb, recon, sino, out, out_mode, st); break;
+    case LK_F16: fwd_launch<K, LK_F16>(A, nb, recon, sino, out, out_mode, st); break;
+    default: fwd_launch<K, LK_U16>(A, nb, recon, sino, out, out_mode, st); break;
   }
 }
 
 }  // namespace
 
-void launch_forward(const IterArgs& A, const float* recon_batch,
+void launch_forward(const IterArgs& A, int nb, const float* recon_batch,
                     const float* sino_batch, float* out, int out_mode,
                     cudaStream_t st) {
   switch (A.K) {
-    case 1: fwd_kind<1>(A, recon_batch, sino_batch, out, out_mode, st); break;
-    case 2: fwd_kind<2>(A, recon_batch, sino_batch, out, out_mode, st); break;
-    case 4: fwd_kind<4>(A, recon_batch, sino_batch, out, out_mode, st); break;
-    case 8: fwd_kind<8>(A, recon_batch, sino_batch, out, out_mode, st); break;
-    default: fwd_kind<16>(A, recon_batch, sino_batch, out, out_mode, st); break;
+    case 1: fwd_kind<1>(A, nb, recon_batch, sino_batch, out, out_mode, st); break;
+    case 2: fwd_kind<2>(A, nb, recon_batch, sino_batch, out, out_mode, st); break;
+    case 4: fwd_kind<4>(A, nb, recon_batch, sino_batch, out, out_mode, st); break;
+    case 8: fwd_kind<8>(A, nb, recon_batch, sino_batch, out, out_mode, st); break;
+    default: fwd_kind<16>(A, nb, recon_batch, sino_batch, out, out_mode, st); break;
   }
 }
 

@@ -302,15 +302,18 @@ void launch_trace_export(const DevGeom& G, const int64_t* offsets, int* idx,
                          float* len, float* len2, cudaStream_t st);
 
 // tg_forward.cu
-void launch_forward(const IterArgs& A, const float* recon_batch,
+// nb consecutive slice batches in one launch (sinogram rows and outputs P*C*K
+// values apart)
+void launch_forward(const IterArgs& A, int nb, const float* recon_batch,
                     const float* sino_batch, float* out, int out_mode,
                     cudaStream_t st);
 // tg_backward.cu
 // per-K instances of launch_backward (tg_backward*.cu)
 #define TG_BACKWARD_DECL(KK)                                                      \
-  void launch_backward_k##KK(const IterArgs& A, int batch, const float* recon_cur, \
-                             float* recon_next, const float* upd, float* rep_num, \
-                             int epi, cudaStream_t st);                            \
+  void launch_backward_k##KK(const IterArgs& A, int first, int nb,                 \
+                             const float* recon_cur, float* recon_next,            \
+                             const float* upd, float* rep_num, int epi,            \
+                             cudaStream_t st);                                     \
   void launch_backward_multi_k##KK(const BackItem* items, int n, int64_t blocks,   \
                                    int dlen_kind, int pen, int fh, int comp,        \
                                    cudaStream_t st);
@@ -319,10 +322,12 @@ TG_BACKWARD_DECL(2)
 TG_BACKWARD_DECL(4)
 TG_BACKWARD_DECL(8)
 #undef TG_BACKWARD_DECL
-void launch_backward_k16(const IterArgs& A, int batch, const float* recon_cur,
+void launch_backward_k16(const IterArgs& A, int first, int nb, const float* recon_cur,
                          float* recon_next, const float* upd, float* rep_num, int epi,
                          cudaStream_t st);
-void launch_backward(const IterArgs& A, int batch, const float* recon_cur,
+// batches first .. first + nb - 1 in one launch, their factors (P*C*K values
+// each) one behind the other at upd
+void launch_backward(const IterArgs& A, int first, int nb, const float* recon_cur,
                      float* recon_next, const float* upd, float* rep_num,
                      int epi, cudaStream_t st);
 // tg_backward_mma*.cu: units first .. first + nunits - 1 of A.F (half_factors

@@ -80,6 +80,9 @@ struct tg_plan {
   // with half_gathers the first one stores halves of the factors, later ones
   // halves of factor - 1 (factor_storage)
   int64_t iters_done = 0;
+  // slice batches per launch of the ray-ordered forward and its
+  // backprojection (plans without the tile-ordered matrix)
+  int launch_nb = 1;
   float* d_upd = nullptr;
   float* d_rep = nullptr;
   float *d_F = nullptr, *d_G = nullptr;
@@ -565,7 +568,7 @@ int build_tiles(tg_plan* p, int* d_nruns) {
 
 int ensure_upd(tg_plan* p) {
   if (p->mma) return TG_OK;  // ensure_factors
-  if (!p->d_upd) TG_TRY(dalloc(p, &p->d_upd, (size_t)p->R * p->K * (p->fp64 ? 2 : 1)));
+  if (!p->d_upd) TG_TRY(dalloc(p, &p->d_upd, (size_t)p->R * p->K * p->launch_nb * (p->fp64 ? 2 : 1)));
   if (p->two && !p->d_upd2) TG_TRY(dalloc(p, &p->d_upd2, (size_t)p->R * p->K));
   return TG_OK;
 }
@@ -1017,6 +1020,11 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
     launch_places(G, M, place, p->st);
     M.place = place;
   }
+  // One launch serves up to 16 slices of a plan without the tile-ordered
+  // matrix: with one slice per pass (the default) a 400-column slice's rays
+  // fill 0.4 of the GPU's warps, and slices in one launch share the matrix
+  // through L2.
+  if (!p->tiles && !p->fp64) p->launch_nb = std::min(p->nb, std::max(1, 16 / p->K));
   // two-stream iterations: tile-staged plans with two or more slice batches
   if (p->tiles && p->nb >= 2 && d.batch_streams != 1) {
     if (cudaStreamCreateWithFlags(&p->st2, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1250,11 +1258,11 @@ int tg_get_recon(tg_plan* p, int alg, float* recon, int on_device) {
   return TG_OK;
 }
 
-// Forward projection of batch b into per-ray values `out` (FP32): the
-// tile-ordered kernel (per-run partial sums, added per ray in path order by
-// the finish kernel) when the plan has the tile-ordered matrix, else the
-// ray-ordered kernel.
-static int run_forward(tg_plan* p, const IterArgs& A0, int b, int out_mode,
+// Forward projection of batches b .. b + nb - 1 into per-ray values `out`
+// (FP32): the tile-ordered kernel (per-run partial sums, added per ray in path
+// order by the finish kernel; nb = 1) when the plan has the tile-ordered
+// matrix, else the ray-ordered kernel.
+static int run_forward(tg_plan* p, const IterArgs& A0, int b, int nb, int out_mode,
                        float* out) {
   const float* src = batch_ptr(p, p->d_recon[p->cur], b * p->K + p->fshift);
   if (p->tiles) {
@@ -1273,9 +1281,22 @@ static int run_forward(tg_plan* p, const IterArgs& A0, int b, int out_mode,
   }
   const IterArgs& A = A0;
   Timed t(p, 0);
-  launch_forward(A, src, p->d_sino + (int64_t)b * p->R * p->K, out, out_mode,
+  launch_forward(A, nb, src, p->d_sino + (int64_t)b * p->R * p->K, out, out_mode,
                  p->st);
   return TG_OK;
+}
+
+// Backprojection of batches b .. b + nb - 1 from the factors at upd.
+static void run_backward(tg_plan* p, const IterArgs& A, int b, int nb, const float* upd,
+                         float* next, float* rep, int epi, cudaStream_t s) {
+  const float* cur = p->d_recon[p->cur];
+  Timed t(p, 1);
+  if (!p->d.backward_staged) {
+    launch_backward(A, b, nb, cur, next, upd, rep, epi, s);
+    return;
+  }
+  for (int i = 0; i < nb; ++i)
+    launch_backward_staged(A, b + i, cur, next, upd + (int64_t)i * p->R * p->K, rep, epi, s);
 }
 
 // Storage of the ratio factors of a fused iteration on a plan that has run
@@ -1344,9 +1365,12 @@ static void issue_units(tg_plan* p, IterArgs A, int mode, bool two, int epi,
 // the caller flips p->cur and counts the iteration).
 // two_streams: the plan's odd slice batches go to its second stream (forked
 // from and joined back into p->st), except while the per-kernel timers run.
+// grouped: several slice batches per launch where the plan allows it (not in
+// a batch of plans, whose branches fill the GPU side by side).
 // after_batch(b, s): called once batch b's backprojection is issued on s.
 static void issue_iteration(tg_plan* p, const IterArgs& A0, int mode, bool two_streams,
-                            const std::function<void(int, cudaStream_t)>& after_batch = {}) {
+                            const std::function<void(int, cudaStream_t)>& after_batch = {},
+                            bool grouped = true) {
   IterArgs A = A0;
   if (p->tiles && p->d.half_gathers) {
     A.half_tile = 1;
@@ -1358,7 +1382,9 @@ static void issue_iteration(tg_plan* p, const IterArgs& A0, int mode, bool two_s
     cudaStreamWaitEvent(p->st2, p->ev_fork, 0);
   }
   if (p->mma) issue_units(p, A, mode, two, EPI_UPDATE, after_batch);
-  for (int b = 0; b < p->nb && !p->mma; ++b) {
+  const int step = grouped ? p->launch_nb : 1;
+  for (int b = 0; b < p->nb && !p->mma; b += step) {
+    const int nb = std::min(step, p->nb - b);
     const bool odd = two && (b & 1);
     const cudaStream_t s = odd ? p->st2 : p->st;
     float* upd = odd ? p->d_upd2 : p->d_upd;
@@ -1372,16 +1398,10 @@ static void issue_iteration(tg_plan* p, const IterArgs& A0, int mode, bool two_s
       Timed t(p, 2);
       launch_fwd_finish(A, p->T, part, p->d_sino + (int64_t)b * p->R * p->K, upd, mode, s);
     } else {
-      run_forward(p, A, b, mode, upd);
+      run_forward(p, A, b, nb, mode, upd);
     }
-    Timed t(p, 1);
-    if (!p->d.backward_staged)
-      launch_backward(A, b, p->d_recon[p->cur], p->d_recon[p->cur ^ 1], upd, nullptr,
-                      EPI_UPDATE, s);
-    else
-      launch_backward_staged(A, b, p->d_recon[p->cur], p->d_recon[p->cur ^ 1], upd,
-                             nullptr, EPI_UPDATE, s);
-    if (after_batch) after_batch(b, s);
+    run_backward(p, A, b, nb, upd, p->d_recon[p->cur ^ 1], nullptr, EPI_UPDATE, s);
+    for (int i = 0; i < nb && after_batch; ++i) after_batch(b + i, s);
   }
   if (two) {
     cudaEventRecord(p->ev_join, p->st2);
@@ -1956,7 +1976,7 @@ extern "C" int tg_batch_iterate(tg_batch* b, const int* algs, const tg_params* p
         const cudaStream_t keep = p->st;
         p->st = b->streams[i % ns];
         const IterArgs A = make_args(p, algs[i], params ? &params[i] : nullptr);
-        issue_iteration(p, A, algs[i] == TG_SIRT ? FWD_SIRT : FWD_RATIO, false);
+        issue_iteration(p, A, algs[i] == TG_SIRT ? FWD_SIRT : FWD_RATIO, false, {}, false);
         p->st = keep;
       }
       for (int s = 0; e == cudaSuccess && s < ns; ++s) {
@@ -2012,15 +2032,10 @@ int tg_reduce(tg_plan* p, int alg, const tg_params* prm) {
     A.half_tile = p->d.half_gathers;
     issue_units(p, A, mode, false, EPI_REPLICA);
   }
-  for (int b = 0; b < p->nb && !p->mma; ++b) {
-    run_forward(p, A, b, mode, p->d_upd);
-    Timed t(p, 1);
-    if (!p->d.backward_staged)
-      launch_backward(A, b, p->d_recon[p->cur], nullptr, p->d_upd, p->d_rep,
-                      EPI_REPLICA, p->st);
-    else
-      launch_backward_staged(A, b, p->d_recon[p->cur], nullptr, p->d_upd,
-                             p->d_rep, EPI_REPLICA, p->st);
+  for (int b = 0; b < p->nb && !p->mma; b += p->launch_nb) {
+    const int nb = std::min(p->launch_nb, p->nb - b);
+    run_forward(p, A, b, nb, mode, p->d_upd);
+    run_backward(p, A, b, nb, p->d_upd, nullptr, p->d_rep, EPI_REPLICA, p->st);
   }
   TG_CUDA(p, cudaGetLastError());
   return TG_OK;
@@ -2118,8 +2133,9 @@ int tg_forward_project(tg_plan* p, int alg, const tg_params* prm, float* sim,
   const bool staged = !on_device && !mapped;
   TG_TRY(stage(p, packed + (staged ? n : 0)));
   const IterArgs A = make_args(p, alg, prm);
-  for (int b = 0; b < p->nb; ++b)
-    run_forward(p, A, b, FWD_SIM, p->d_stage + (int64_t)b * p->R * p->K);
+  for (int b = 0; b < p->nb; b += p->launch_nb)
+    run_forward(p, A, b, std::min(p->launch_nb, p->nb - b), FWD_SIM,
+                p->d_stage + (int64_t)b * p->R * p->K);
   float* dst = on_device ? sim : mapped ? mapped : p->d_stage + packed;
   launch_sino_unpack(p->d_stage, dst, p->P, p->S, p->C, p->K, p->st);
   TG_CUDA(p, cudaGetLastError());
@@ -2207,9 +2223,9 @@ extern "C" int tg_reduce_slice_noalloc(tg_plan* p, int alg,
   A.vshift = 0;
   A.fshift = 0;
   A.nslots = 1;
-  launch_forward(A, recon, sino, factors, alg == TG_SIRT ? FWD_SIRT : FWD_RATIO,
+  launch_forward(A, 1, recon, sino, factors, alg == TG_SIRT ? FWD_SIRT : FWD_RATIO,
                  p->st);
-  launch_backward(A, 0, recon, nullptr, factors, num, EPI_REPLICA, p->st);
+  launch_backward(A, 0, 1, recon, nullptr, factors, num, EPI_REPLICA, p->st);
   TG_CUDA(p, cudaGetLastError());
   return TG_OK;
 }
