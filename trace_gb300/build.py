@@ -22,7 +22,7 @@ SOURCES = [
     "tg_backward_k8.cu", "tg_backward_k16.cu", "tg_backward_mma.cu",
     "tg_backward_mma_split.cu", "tg_backward_mma_u16.cu", "tg_backward_mma_bf16.cu",
     "tg_backward_mma_f32.cu", "tg_backward_staged.cu", "tg_iter.cu", "tg_fp64.cu",
-    "tg_tiles.cu", "tg_plan.cu",
+    "tg_tiles.cu", "tg_strips.cu", "tg_plan.cu",
 ]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

@@ -108,6 +108,40 @@ struct TileMatrixDev {
   const uint32_t* tcode;    // 8 x 4-bit step codes per word per lane
 };
 
+// Strip-ordered forward matrix (tg_strips.cu). The slope of a ray is its shift
+// in pixels per row (class 0: rows are pixel rows; class 1: pixel columns);
+// positions of a group of angles lie within mid x d +- half x |d| at d rows
+// from a chunk's middle, and a ray's pixels in a row within +- ext.
+constexpr int kStripCols = 28;  // pixels staged per row by a block
+struct StripSlopes {
+  float mid, half, ext;
+};
+struct StripExc {
+  int ray, idx, code, pad;
+};
+struct StripDev {
+  int P, R, nchunks;       // rows per chunk
+  uint32_t rmul;           // m / R = umulhi(m, rmul), as TileDiv's
+  int strip0, nstrips;     // first strip's index; strips (a multiple of 4)
+  int nblk16;              // blocks of 16 angles of one class
+  int64_t nbundles;        // nchunks x nblk16 x nstrips x 4 quads
+  const int* cls;          // [P]
+  const int* place;        // [P] block x 16 + quad x 4 + angle of the quad
+  const int64_t* alpha;    // [nchunks][P] position of column 0 at the chunk's
+                           // middle row, in 2^-20 pixels
+  const int64_t* sigma;    // [P] and its step per column (at least a pixel)
+  const int* cls16;        // [nblk16]
+  const StripSlopes* blk16;  // [nblk16]
+  const StripSlopes* quad;   // [nblk16 * 4]
+  const uint2* codes;      // [bundle][R / 4][16 rays][4 rows] even and odd
+                           // pixels' pairs of 16-bit codes
+  const uint32_t* meta;    // [bundle][R / 4][8][2]
+  const int* exc_first;    // [P*C + 1] exceptions per ray, or nullptr
+  const StripExc* exc;
+  const uint8_t* grazed;   // [C*C] 1: a ray's zero-length segment lies in the pixel
+  int* bad;                // a crossed pixel's half is not finite
+};
+
 // Which per-ray value the forward kernel stores.
 enum FwdOut { FWD_SIRT = 0, FWD_RATIO = 1, FWD_SIM = 2 };
 // What the backward kernel does with its per-pixel sums.
@@ -440,6 +474,24 @@ void launch_backward_multi(const BackItem* items, int n, int64_t blocks, int K,
                            int dlen_kind, int pen, int fh, int comp, cudaStream_t st);
 // blocks (of 256 threads) a plan's backprojection launch uses
 int64_t backward_blocks(const IterArgs& A);
+// tg_strips.cu
+// the rays' pixel indices and length codes (16-bit storage) in the layout of
+// the ray-ordered matrix
+void launch_strips_trace(const DevGeom& G, const MatrixDev& M, int* ridx, uint16_t* rlen,
+                         cudaStream_t st);
+void launch_strips_fill(const DevGeom& G, const MatrixDev& M, const StripDev& S, uint2* codes,
+                        uint32_t* meta, uint8_t* grazed, StripExc* exc, int exc_cap, int* nexc,
+                        cudaStream_t st);
+// U (32 or 64) slices from slice `first`: their halves into img ([pixel][U]),
+// then every bundle's sums into part ([bundle][16][U]); reset: the flags and
+// largest factors of their batches too
+void launch_strips_forward(const IterArgs& A, const StripDev& S, int first, int U,
+                           const float* recon, __half* img, float* part, int reset,
+                           cudaStream_t st);
+// their per-ray values: factors into A.F, or the sums ([S/K][P*C][K]) into sim
+void launch_strips_finish(const IterArgs& A, const StripDev& S, int first, int U,
+                          const __half* img, const float* part, const float* sino, float* sim,
+                          int out_mode, cudaStream_t st);
 // tg_iter.cu
 void launch_fg(const IterArgs& A, const float* recon, const float* W, float* F,
                float* Gv, cudaStream_t st);

@@ -68,6 +68,12 @@ struct tg_plan {
   int unit = 0, nunits = 0, group_units = 1;  // slices per unit, units, units per group
   int* d_flags = nullptr;
   cudaEvent_t ev_meet = nullptr, ev_group[2] = {nullptr, nullptr};
+  // strip-ordered forward (in place of the tile-ordered one): a group's halves
+  // of the reconstruction and bundle sums
+  bool strips = false;
+  StripDev St{};
+  __half* d_simg = nullptr;
+  float* d_spart = nullptr;
   // FP64 mode: double state, factors, total lengths and SIRT's a2
   bool fp64 = false;
   double *d_ra2d = nullptr, *d_W64 = nullptr;
@@ -566,6 +572,214 @@ int build_tiles(tg_plan* p, int* d_nruns) {
   return TG_OK;
 }
 
+// Chunks, strips and angle groups of the strip-ordered forward matrix for the
+// plan's geometry, its tables on the device and its codes: TG_OK with
+// p->strips set, or left unset where the geometry or memory does not allow it
+// (the tile-ordered matrix is built then).
+struct StripTables {
+  int R = 0;
+  int64_t entries = 0;  // of the ray-ordered matrix
+  std::vector<int> cls, place, cls16;
+  std::vector<int64_t> sigma;
+  std::vector<double> n0, kappa;  // position of column 0 at row 0, slope
+  std::vector<StripSlopes> blk16, quad;
+};
+
+bool strip_tables(const tg_plan* p, const std::vector<float>& sn, const std::vector<float>& cs,
+                  StripTables& T) {
+  const int P = p->P, C = p->C;
+  T.cls.resize(P);
+  T.place.resize(P);
+  T.sigma.resize(P);
+  T.n0.resize(P);
+  T.kappa.resize(P);
+  const double off = (1.0 - C) / 2.0 + (double)p->mov, h = C / 2.0;
+  for (int a = 0; a < P; ++a) {
+    const double s = sn[a], c = cs[a];
+    if (!std::isfinite(s) || !std::isfinite(c) || std::fabs(s * s + c * c - 1.0) > 1e-3)
+      return false;
+    const bool col = std::fabs(c) > std::fabs(s);
+    T.cls[a] = col;
+    // rows: x = y cot - t / sin; columns: y = x tan + t / cos (centred)
+    T.kappa[a] = col ? s / c : c / s;
+    const double step = col ? 1.0 / c : -1.0 / s;
+    int64_t f = llrint(step * 1048576.0);
+    if (f >= 0 && f < 1048576) f = 1048576;
+    if (f < 0 && f > -1048576) f = -1048576;
+    T.sigma[a] = f;
+    T.n0[a] = h + step * off - T.kappa[a] * h;
+  }
+  // blocks of 16 consecutive angles of one class
+  double half4 = 0, part16 = 0;
+  auto slopes = [&](int a0, int a1, double& half) {
+    double lo = T.kappa[a0], hi = lo, ext = 0;
+    for (int a = a0; a < a1; ++a) {
+      lo = std::min(lo, T.kappa[a]);
+      hi = std::max(hi, T.kappa[a]);
+      ext = std::max(ext, std::fabs(T.kappa[a]));
+    }
+    half = (hi - lo) / 2;
+    // half a row of slope, and 3/8 for the reference's float jitter
+    return StripSlopes{(float)((hi + lo) / 2), (float)half, (float)(ext / 2 + 0.375)};
+  };
+  for (int a0 = 0; a0 < P;) {
+    int a1 = a0 + 1;
+    while (a1 < P && a1 - a0 < 16 && T.cls[a1] == T.cls[a0]) ++a1;
+    double h16 = 0, hq[4] = {0, 0, 0, 0};
+    StripSlopes b = slopes(a0, a1, h16);
+    b.ext += 0.02f;  // at most every quad's, rounding included
+    T.blk16.push_back(b);
+    T.cls16.push_back(T.cls[a0]);
+    for (int q = 0; q < 4; ++q) {
+      const int q0 = std::min(a0 + 4 * q, a1 - 1), q1 = std::max(q0 + 1, std::min(a0 + 4 * q + 4, a1));
+      T.quad.push_back(slopes(q0, q1, hq[q]));
+      half4 = std::max(half4, hq[q]);
+      part16 = std::max(part16, h16 - hq[q]);
+    }
+    for (int a = a0; a < a1; ++a) T.place[a] = ((int)T.blk16.size() - 1) * 16 + (a - a0);
+    a0 = a1;
+  }
+  // Rows per chunk: over half a chunk a quad's window (4 pixels of strip, the
+  // slopes' spread, a row's slope and the jitter) stays within 8 pixels, and
+  // the four strips' and quads' windows within the staged ones.
+  int R = 256;
+  for (; R >= 32; R -= 8)
+    if (R * half4 <= 1.2 && R * part16 <= kStripCols - 8 - 12 - 1.2) break;
+  if (R < 32) return false;
+  const int n = (C + R - 1) / R;  // chunks of about equal size
+  T.R = ((C + n - 1) / n + 7) / 8 * 8;
+  return true;
+}
+
+int build_strips(tg_plan* p, const StripTables& T) {
+  const int P = p->P, C = p->C;
+  std::vector<void*> got;  // kept allocations, freed when the build gives up
+  std::vector<size_t> size;
+  auto give_up = [&]() {
+    for (size_t i = 0; i < got.size(); ++i) dfree(p, got[i], size[i]);
+    p->d_simg = nullptr;
+    p->d_spart = nullptr;
+    p->err.clear();
+    return TG_OK;
+  };
+  auto keep = [&](auto** ptr, size_t n, bool zero) {
+    if (dalloc(p, ptr, n, zero) != TG_OK) return false;
+    got.push_back((void*)*ptr);
+    size.push_back(n * sizeof(**ptr));
+    return true;
+  };
+  StripDev S{};
+  S.P = P;
+  S.R = T.R;
+  S.rmul = make_tile_div(T.R).m;
+  S.nchunks = (C + T.R - 1) / T.R;
+  S.strip0 = -(T.R / 2 + 8) / 4 - 1;
+  S.nstrips = ((C + T.R + 16) / 4 + 4 + 3) / 4 * 4;
+  S.nblk16 = (int)T.blk16.size();
+  S.nbundles = (int64_t)S.nchunks * S.nblk16 * S.nstrips * 4;
+  std::vector<int64_t> alpha((size_t)S.nchunks * P);
+  for (int j = 0; j < S.nchunks; ++j)
+    for (int a = 0; a < P; ++a)
+      alpha[(size_t)j * P + a] =
+          llrint((T.n0[a] + T.kappa[a] * ((j + 0.5) * T.R)) * 1048576.0);
+  int *cls, *place, *cls16;
+  int64_t *al, *sg;
+  StripSlopes *b16, *quad;
+  uint2* codes;
+  uint32_t* meta;
+  uint8_t* grazed;
+  const size_t nsteps = (size_t)S.nbundles * (T.R / 4);
+  const size_t U = std::min(p->group_units * p->unit, p->S) <= 32 ? 32 : 64;
+  StripExc* exc = nullptr;
+  int* nexc = nullptr;
+  constexpr int kCap = 1 << 20;
+  if (!keep(&cls, P, false) || !keep(&place, P, false) || !keep(&cls16, S.nblk16, false) ||
+      !keep(&al, alpha.size(), false) || !keep(&sg, P, false) || !keep(&b16, S.nblk16, false) ||
+      !keep(&quad, T.quad.size(), false) || !keep(&S.bad, 1, true) ||
+      !keep(&grazed, p->g2, true) || !keep(&codes, nsteps * 64, true) ||
+      !keep(&meta, nsteps * 16, false) ||
+      !keep(&p->d_simg, U * p->g2, false) || !keep(&p->d_spart, U * S.nbundles * 16, false))
+    return give_up();
+  if (dalloc(p, &exc, kCap) != TG_OK) return give_up();
+  if (dalloc(p, &nexc, 1, true) != TG_OK) {
+    dfree(p, exc, kCap * sizeof(StripExc));
+    return give_up();
+  }
+  auto put = [&](void* d, const void* h, size_t n) {
+    cudaMemcpyAsync(d, h, n, cudaMemcpyHostToDevice, p->st);
+  };
+  put(cls, T.cls.data(), P * 4);
+  put(place, T.place.data(), P * 4);
+  put(cls16, T.cls16.data(), S.nblk16 * 4);
+  put(al, alpha.data(), alpha.size() * 8);
+  put(sg, T.sigma.data(), P * 8);
+  put(b16, T.blk16.data(), T.blk16.size() * sizeof(StripSlopes));
+  put(quad, T.quad.data(), T.quad.size() * sizeof(StripSlopes));
+  cudaMemsetAsync(meta, 0x44, nsteps * 64, p->st);
+  S.cls = cls;
+  S.place = place;
+  S.alpha = al;
+  S.sigma = sg;
+  S.cls16 = cls16;
+  S.blk16 = b16;
+  S.quad = quad;
+  S.codes = codes;
+  S.meta = meta;
+  S.grazed = grazed;
+  // a plan whose rays have stray steps keeps no ray-ordered matrix: one for the
+  // fill alone
+  MatrixDev M = p->M;
+  int* ridx = nullptr;
+  uint16_t* rlen = nullptr;
+  bool ok = true;
+  if (!M.rlen) {
+    ok = dalloc(p, &ridx, (size_t)T.entries) == TG_OK && dalloc(p, &rlen, (size_t)T.entries) == TG_OK;
+    if (ok) launch_strips_trace(p->G, M, ridx, rlen, p->st);
+    M.ridx = ridx;
+    M.rlen = rlen;
+  }
+  if (ok) launch_strips_fill(p->G, M, S, codes, meta, grazed, exc, kCap, nexc, p->st);
+  int n = 0;
+  cudaMemcpyAsync(&n, nexc, 4, cudaMemcpyDeviceToHost, p->st);
+  int rc = TG_OK;
+  if (cudaStreamSynchronize(p->st) != cudaSuccess)
+    rc = fail(p, TG_E_CUDA, "filling the strip-ordered matrix failed");
+  ok = ok && rc == TG_OK && n <= kCap;
+  if (ok && n > 0) {
+    // per ray, in a fixed order
+    std::vector<StripExc> e(n);
+    std::vector<int> first((size_t)p->R + 1, 0);
+    cudaMemcpy(e.data(), exc, n * sizeof(StripExc), cudaMemcpyDeviceToHost);
+    std::sort(e.begin(), e.end(), [](const StripExc& x, const StripExc& y) {
+      return x.ray != y.ray ? x.ray < y.ray : x.idx != y.idx ? x.idx < y.idx : x.code < y.code;
+    });
+    for (const StripExc& x : e) ++first[(size_t)x.ray + 1];
+    for (int64_t r = 0; r < p->R; ++r) first[r + 1] += first[r];
+    int* d_first = nullptr;
+    StripExc* d_exc = nullptr;
+    if (keep(&d_first, first.size(), false) && keep(&d_exc, (size_t)n, false)) {
+      cudaMemcpy(d_first, first.data(), first.size() * 4, cudaMemcpyHostToDevice);
+      cudaMemcpy(d_exc, e.data(), n * sizeof(StripExc), cudaMemcpyHostToDevice);
+      S.exc_first = d_first;
+      S.exc = d_exc;
+    } else {
+      ok = false;
+    }
+  }
+  dfree(p, exc, kCap * sizeof(StripExc));
+  dfree(p, nexc, sizeof(int));
+  if (ridx) dfree(p, ridx, (size_t)T.entries * 4);
+  if (rlen) dfree(p, rlen, (size_t)T.entries * 2);
+  if (rc != TG_OK) return rc;
+  if (!ok) return give_up();
+  p->St = S;
+  p->strips = p->tiles = true;
+  p->info.tile_runs = p->R * S.nchunks;
+  p->info.partial_slots = S.nbundles * 16;
+  p->info.tile_bytes = (int64_t)nsteps * (64 * 8 + 16 * 4);
+  return TG_OK;
+}
+
 int ensure_upd(tg_plan* p) {
   if (p->mma) return TG_OK;  // ensure_factors
   if (!p->d_upd) TG_TRY(dalloc(p, &p->d_upd, (size_t)p->R * p->K * p->launch_nb * (p->fp64 ? 2 : 1)));
@@ -992,10 +1206,6 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
   if (p->fp64) launch_weights64(G, M, p->d_W64, p->st);
   p->info.window_exceptions = (int64_t)nexc;
   (void)counters[1];
-  if (d.forward_tiles && (rc = build_tiles(p, d_nruns))) {
-    if (p->err.empty()) p->err = "building the tile-ordered forward matrix failed";
-    return bail(rc);
-  }
   // The backprojection runs on the tensor cores for half-gather plans with
   // 16-bit lengths (f16 in the backward matrix), and for FP32 operands at 8
   // slices per pass. A larger unit of slices spreads a tile's A operand over
@@ -1003,7 +1213,7 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
   // 0.61 of 16, 0.39 of 32), but a small grid has too few blocks to fill the
   // GPU with, so the unit is the largest one that leaves two blocks per SM.
   // Groups of units (64 slices) are one launch.
-  p->mma = p->tiles && !d.backward_staged && !d.compensated &&
+  p->mma = d.forward_tiles && !d.backward_staged && !d.compensated &&
            (d.half_gathers ? M.dlen_kind == LK_F16 : p->K == 8);
   if (p->mma) {
     int sms = 0, dev = 0;
@@ -1020,13 +1230,29 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
     launch_places(G, M, place, p->st);
     M.place = place;
   }
+  // Many slices, 16-bit codes and angles close enough for the strips (32 rows
+  // per chunk and more): the strip-ordered forward. Its codes take 9 bytes per
+  // ray and row where the tile stream takes 3, but are read once per 32 or 64
+  // slices. 1024 x 1024 x 720, forward and finish: 32 slices 4.1 ms in tiles,
+  // 2.9 in strips; 64 slices 8.2 and 4.6; 24 slices 3.1 and 2.9, which is not
+  // worth the memory. A plan that traces on the fly, to save memory, keeps the
+  // tiles too.
+  if (p->mma && d.half_gathers && p->len_kind == TG_LEN_U16 && !otf && p->S >= 32) {
+    StripTables T;
+    T.entries = entries;
+    if (strip_tables(p, sn, cs, T) && (rc = build_strips(p, T))) return bail(rc);
+  }
+  if (d.forward_tiles && !p->strips && (rc = build_tiles(p, d_nruns))) {
+    if (p->err.empty()) p->err = "building the tile-ordered forward matrix failed";
+    return bail(rc);
+  }
   // One launch serves up to 16 slices of a plan without the tile-ordered
   // matrix: with one slice per pass (the default) a 400-column slice's rays
   // fill 0.4 of the GPU's warps, and slices in one launch share the matrix
   // through L2.
   if (!p->tiles && !p->fp64) p->launch_nb = std::min(p->nb, std::max(1, 16 / p->K));
   // two-stream iterations: tile-staged plans with two or more slice batches
-  if (p->tiles && p->nb >= 2 && d.batch_streams != 1) {
+  if (p->tiles && !p->strips && p->nb >= 2 && d.batch_streams != 1) {
     if (cudaStreamCreateWithFlags(&p->st2, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming) != cudaSuccess ||
@@ -1311,6 +1537,20 @@ static int half_factors_next(const tg_plan* p, int mode) {
   return factor_storage(p, mode, p->iters_done);
 }
 
+// Strip-ordered forward projection of group g's slices: their factors into
+// A.F, or their ray sums ([S/K][P*C][K]) into sim.
+static void run_strips(tg_plan* p, const IterArgs& A, int g, int mode, float* sim) {
+  const int per_group = p->group_units * p->unit, first = g * per_group;
+  const int U = std::min(per_group, p->S - first) <= 32 ? 32 : 64;
+  {
+    Timed t(p, 0);
+    launch_strips_forward(A, p->St, first, U, p->d_recon[p->cur], p->d_simg, p->d_spart,
+                          sim == nullptr, p->st);
+  }
+  Timed t(p, 2);
+  launch_strips_finish(A, p->St, first, U, p->d_simg, p->d_spart, p->d_sino, sim, mode, p->st);
+}
+
 // The iteration of a plan with the tensor-core backprojection: every batch's
 // forward projection and finish, and per group of units one backprojection.
 // two: odd batches and odd groups run on the second stream; a group's
@@ -1328,7 +1568,8 @@ static void issue_units(tg_plan* p, IterArgs A, int mode, bool two, int epi,
     const int b0 = g * per_group / p->K;
     const int b1 = std::min(p->nb, (g + 1) * per_group / p->K);
     if (two && g >= 2) cudaStreamWaitEvent(st[(g + 1) & 1], p->ev_group[g & 1], 0);
-    for (int b = b0; b < b1; ++b) {
+    if (p->strips) run_strips(p, A, g, mode, nullptr);
+    for (int b = b0; b < b1 && !p->strips; ++b) {
       const int odd = two ? b & 1 : 0;
       float* part = odd ? p->d_part2 : p->d_part;
       {
@@ -1580,7 +1821,7 @@ struct tg_batch {
 namespace {
 
 bool multi_eligible(const tg_plan* p) {
-  return !p->fp64 && p->tiles && !p->d.backward_staged && p->d.mode == TG_MODE_FAST &&
+  return !p->fp64 && p->tiles && !p->strips && !p->d.backward_staged && p->d.mode == TG_MODE_FAST &&
          p->len_kind == TG_LEN_U16 && p->nunits <= 2 * p->group_units;
 }
 
@@ -1948,7 +2189,8 @@ extern "C" int tg_batch_iterate(tg_batch* b, const int* algs, const tg_params* p
     // float factors are split
     const int mode = algs[i] == TG_SIRT ? FWD_SIRT : FWD_RATIO;
     const bool split = p->F[half_factors_next(p, mode) != FACT_F32].split != nullptr;
-    b->last_launches += p->mma ? p->nb * 2 + (p->nunits + p->group_units - 1) / p->group_units *
+    const int fwd = p->strips ? 4 * ((p->nunits + p->group_units - 1) / p->group_units) : p->nb * 2;
+    b->last_launches += p->mma ? fwd + (p->nunits + p->group_units - 1) / p->group_units *
                                                 (split ? 2 : 1)
                                : p->nb * (p->tiles ? 3 : 2);
   }
@@ -2133,7 +2375,9 @@ int tg_forward_project(tg_plan* p, int alg, const tg_params* prm, float* sim,
   const bool staged = !on_device && !mapped;
   TG_TRY(stage(p, packed + (staged ? n : 0)));
   const IterArgs A = make_args(p, alg, prm);
-  for (int b = 0; b < p->nb; b += p->launch_nb)
+  const int groups = p->strips ? (p->nunits + p->group_units - 1) / p->group_units : 0;
+  for (int g = 0; g < groups; ++g) run_strips(p, A, g, FWD_SIM, p->d_stage);
+  for (int b = 0; b < p->nb && !p->strips; b += p->launch_nb)
     run_forward(p, A, b, std::min(p->launch_nb, p->nb - b), FWD_SIM,
                 p->d_stage + (int64_t)b * p->R * p->K);
   float* dst = on_device ? sim : mapped ? mapped : p->d_stage + packed;
