@@ -19,7 +19,7 @@ OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libtrace_gb300.so")
 SOURCES = [
     "tg_trace.cu", "tg_forward.cu", "tg_backward.cu", "tg_backward_k4.cu",
-    "tg_backward_k8.cu", "tg_backward_k16.cu", "tg_backward_mma.cu",
+    "tg_backward_k8.cu", "tg_backward_k16.cu", "tg_backward_planes.cu", "tg_backward_mma.cu",
     "tg_backward_mma_split.cu", "tg_backward_mma_u16.cu", "tg_backward_mma_bf16.cu",
     "tg_backward_mma_f32.cu", "tg_backward_staged.cu", "tg_iter.cu", "tg_fp64.cu",
     "tg_tiles.cu", "tg_strips.cu", "tg_plan.cu",

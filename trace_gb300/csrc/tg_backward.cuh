@@ -1,8 +1,9 @@
 // Backprojection (pixel-driven) with the algorithms' UpdateRecon fused into
-// its epilogue: exact mode, plans without the tile-staged forward, fewer than
-// 8 slices per pass with FP32 operands, compensated sums and the
+// its epilogue: exact mode, plans without the tile-staged forward, few slices,
+// fewer than 8 slices per pass with FP32 operands, compensated sums and the
 // allocation-free entry point. The other plans' runs on the tensor cores
-// (tg_backward_mma.cuh).
+// (tg_backward_mma.cuh); one slice per pass without compensated sums is
+// tg_backward_planes.cu's.
 //
 // One thread per pixel, one warp per 32-pixel tile (8x4 by default; 16x2
 // or 4x8 as the plan chooses), eight tiles per block.
@@ -163,6 +164,40 @@ __device__ __forceinline__ void accumulate(float (&acc)[K], const float (&rf)[K]
   } else {
     fma_slices<K>(acc, l, u.v);
   }
+}
+
+// The algorithm's update of slice s at pixel (x, y) from its sum (or, EPI_REPLICA,
+// the sum itself); Wp: the pixel's total length.
+template <int K, bool EXACT, bool PEN>
+__device__ __forceinline__ void update_pixel(const IterArgs& A, int s, int x, int y, float num,
+                                             float Wp, const float* __restrict__ cur,
+                                             float* __restrict__ next,
+                                             float* __restrict__ rep_num, int epi) {
+  const int g = A.G.C;
+  const int64_t g2 = (int64_t)g * g, p = (int64_t)y * g + x;
+  if (epi == EPI_REPLICA) {
+    rep_num[(int64_t)s * g2 + p] = num;
+    return;
+  }
+  const int ts = s + A.vshift;
+  const int64_t at = slot_addr(ts, p, g2, K);
+  const float old = cur[at];
+  float nv;
+  if constexpr (!PEN) {
+    nv = A.alg == 0 ? fadd(old, fdiv(num, Wp)) : fmul(old, fdiv(num, Wp));
+  } else {
+    int up = 0, down = 0;
+    if (A.alg == 3) apmlr_axial(A, s, &up, &down);
+    float F, Gv;
+    penalty_fg(A.alg == 3, A.pw, x, y, g, up, down,
+               [&](int dx, int dy, int dz) {
+                 return cur[slot_addr(ts + dz, p + dx + (int64_t)dy * g, g2, K)];
+               },
+               F, Gv);
+    Gv = fadd(Gv, Wp);
+    nv = EXACT ? penalised_root(F, Gv, num) : penalised_root_stable(F, Gv, num);
+  }
+  next[at] = nv;
 }
 
 // Resident blocks per SM for each variant: compensated sums keep two more
@@ -342,47 +377,23 @@ __device__ __forceinline__ void backward_block(const IterArgs& A, int batch, int
   for (int j = 0; j < K; ++j) {
     const int s = batch * K + j;
     if (s >= A.S) break;
-    const float num = acc[j];
-    if (epi == EPI_REPLICA) {
-      rep_num[(int64_t)s * g2 + p] = num;
-      continue;
-    }
-    const int ts = s + A.vshift;
-    const int64_t at = slot_addr(ts, p, g2, K);
-    const float old = cur[at];
-    float nv;
-    if constexpr (!PEN) {
-      nv = A.alg == 0 ? fadd(old, fdiv(num, Wp)) : fmul(old, fdiv(num, Wp));
-    } else {
-      int up = 0, down = 0;
-      if (A.alg == 3) apmlr_axial(A, s, &up, &down);
-      float F, Gv;
-      penalty_fg(A.alg == 3, A.pw, x, y, g, up, down,
-                 [&](int dx, int dy, int dz) {
-                   return cur[slot_addr(ts + dz, p + dx + (int64_t)dy * g, g2, K)];
-                 },
-                 F, Gv);
-      Gv = fadd(Gv, Wp);
-      nv = EXACT ? penalised_root(F, Gv, num) : penalised_root_stable(F, Gv, num);
-    }
-    next[at] = nv;
+    update_pixel<K, EXACT, PEN>(A, s, x, y, acc[j], Wp, cur, next, rep_num, epi);
   }
 }
 
 template <int K, int LK, bool EXACT, bool PEN, bool FH, bool COMP>
 __global__ void __launch_bounds__(kBlock, (min_blocks<K, COMP>()))
-    k_backward(IterArgs A, int first, int nb, const float* __restrict__ cur,
+    k_backward(IterArgs A, int first, const float* __restrict__ cur,
                float* __restrict__ next, const float* __restrict__ upd,
                float* __restrict__ rep_num, int epi) {
   __shared__ float4 s_coef[kCoefChunk];
   // batches first .. first + nb - 1, each with its factors behind the other:
   // consecutive blocks take the same pixels of all of them, so that they read
   // a piece of the matrix while it is in L2
-  const int blk = blockIdx.x / nb, b = blockIdx.x - blk * nb;
-  const float* u = FH ? reinterpret_cast<const float*>(
-                            reinterpret_cast<const __half*>(upd) + b * ((int64_t)A.G.P * A.G.C * K))
-                      : upd + b * ((int64_t)A.G.P * A.G.C * K);
-  backward_block<K, LK, EXACT, PEN, FH, COMP>(A, first + b, blk, cur, next, u, rep_num, epi,
+  // (tile-staged plans, which half factors imply, launch one batch)
+  const int b = FH ? 0 : blockIdx.x;
+  const float* u = FH ? upd : upd + b * ((int64_t)A.G.P * A.G.C * K);
+  backward_block<K, LK, EXACT, PEN, FH, COMP>(A, first + b, grid_block(), cur, next, u, rep_num, epi,
                                               s_coef);
 }
 
@@ -398,9 +409,10 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<K, COMP>()))
                                               s_coef);
 }
 
-// Multi-plan launches for plans with 16-bit fixed-point lengths: compensated
-// sums (backward matrix u16 codes, or IEEE halves with half gathers), or FP32
-// operands at fewer than 8 slices per pass; the rest is tg_backward_mma.cuh's.
+// Multi-plan launches for plans with 16-bit fixed-point lengths (backward
+// matrix u16 codes, or IEEE halves with half gathers): compensated sums, few
+// slices, or FP32 operands at fewer than 8 slices per pass; the rest is
+// tg_backward_mma.cuh's.
 template <int K>
 void back_multi(const BackItem* items, int n, int64_t blocks, int dlen_kind, int pen,
                 int fh, int comp, cudaStream_t st) {
@@ -411,7 +423,11 @@ void back_multi(const BackItem* items, int n, int64_t blocks, int dlen_kind, int
     else                                                                                 \
       k_backward_multi<K, LKK, false, FHH, CP><<<(unsigned)blocks, kBlock, 0, st>>>(items, n); \
   } while (0)
-  if (!comp) {
+  if (!comp && dlen_kind == LK_F16) {
+    if constexpr (K <= 4) {
+      if (fh) TG_BM(LK_F16, true, false); else TG_BM(LK_F16, false, false);
+    }
+  } else if (!comp) {
     if constexpr (K < 8) TG_BM(LK_U16, false, false);
   } else if (dlen_kind == LK_F16) {
     if (fh) TG_BM(LK_F16, true, true); else TG_BM(LK_F16, false, true);
@@ -424,14 +440,24 @@ void back_multi(const BackItem* items, int n, int64_t blocks, int dlen_kind, int
 template <int K, int LK>
 void back_launch(const IterArgs& A, int first, int nb, const float* cur, float* next,
                  const float* upd, float* rep_num, int epi, cudaStream_t st) {
-  const int blocks = (A.M.ntiles + kWarps - 1) / kWarps * nb;
+  const dim3 blocks = batch_grid((A.M.ntiles + kWarps - 1) / kWarps, nb);
   const bool pen = A.alg >= 2;
 #define TG_BACK(E, PN, FH, CP)                                                        \
-  k_backward<K, LK, E, PN, FH, CP><<<blocks, kBlock, 0, st>>>(A, first, nb, cur, next, \
+  k_backward<K, LK, E, PN, FH, CP><<<blocks, kBlock, 0, st>>>(A, first, cur, next, \
                                                              upd, rep_num, epi)
   // compensated sums: up to 8 slices per pass (plan creation checks)
   constexpr bool kComp = K <= 8;
-  if (A.exact) {
+  if (K == 1 && !A.comp) {
+    launch_backward_planes(A, first, nb, cur, next, upd, rep_num, epi, st);
+    return;
+  }
+  if constexpr (K == 1) {
+    if (A.half_factors) {
+      if (pen) TG_BACK(false, true, true, true); else TG_BACK(false, false, true, true);
+    } else {
+      if (pen) TG_BACK(false, true, false, true); else TG_BACK(false, false, false, true);
+    }
+  } else if (A.exact) {
     if (pen) TG_BACK(true, true, false, false); else TG_BACK(true, false, false, false);
   } else if (kComp && A.comp) {
     if (A.half_factors) {
@@ -440,9 +466,9 @@ void back_launch(const IterArgs& A, int first, int nb, const float* cur, float* 
       if (pen) TG_BACK(false, true, false, kComp); else TG_BACK(false, false, false, kComp);
     }
   } else if (A.half_factors) {
-    // float lengths only: half factors with 16-bit lengths are
-    // tg_backward_mma.cuh's
-    if constexpr (LK == LK_F32) {
+    // half factors with 16-bit lengths are tg_backward_mma.cuh's but for plans
+    // of few slices
+    if constexpr (LK == LK_F32 || (LK == LK_F16 && K <= 4)) {
       if (pen) TG_BACK(false, true, true, false); else TG_BACK(false, false, true, false);
     }
   } else {

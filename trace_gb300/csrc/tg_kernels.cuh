@@ -220,6 +220,9 @@ struct IterArgs {
   // compensated (Kahan) summation of the ray and pixel sums (fast mode,
   // tile-staged forward, L1 backprojection)
   int comp;
+  // one slice per pass: room for a launch's planes with rows and columns
+  // exchanged, or null
+  float* turned;
 };
 
 // Work items of the launches that serve many plans at once (tg_batch): one
@@ -335,6 +338,15 @@ void launch_weights(const DevGeom& G, const MatrixDev& M, int exact, float* W,
 void launch_trace_export(const DevGeom& G, const int64_t* offsets, int* idx,
                          float* len, float* len2, cudaStream_t st);
 
+// Grid of `blocks` blocks for each of nb slice batches, those of one block
+// next to one another: the batch is blockIdx.x (uniform, without a division),
+// the block grid_block().
+inline dim3 batch_grid(int64_t blocks, int nb) {
+  const unsigned y = (unsigned)(blocks < 65535 ? blocks : 65535);
+  return dim3((unsigned)nb, y, (unsigned)((blocks + y - 1) / y));
+}
+__device__ __forceinline__ int grid_block() { return (int)(blockIdx.z * gridDim.y + blockIdx.y); }
+
 // tg_forward.cu
 // nb consecutive slice batches in one launch (sinogram rows and outputs P*C*K
 // values apart)
@@ -364,6 +376,17 @@ void launch_backward_k16(const IterArgs& A, int first, int nb, const float* reco
 void launch_backward(const IterArgs& A, int first, int nb, const float* recon_cur,
                      float* recon_next, const float* upd, float* rep_num,
                      int epi, cudaStream_t st);
+// tg_backward_planes.cu: the same at one slice per pass, sums not compensated
+void launch_backward_planes(const IterArgs& A, int first, int n, const float* cur, float* next,
+                            const float* upd, float* rep_num, int epi, cudaStream_t st);
+// Slices (at most four) a thread of a launch over n slices takes at one slice
+// per pass, where one slice's launch has `warps` warps: four, two or one, the
+// first with need4 (need2) warps left, evened out over the groups.
+inline int planes_per_thread(int64_t warps, int n, int64_t need4, int64_t need2) {
+  const int most = warps * ((n + 3) / 4) >= need4 ? 4 : warps * ((n + 1) / 2) >= need2 ? 2 : 1;
+  const int groups = (n + most - 1) / most;
+  return (n + groups - 1) / groups;
+}
 // tg_backward_mma*.cu: units first .. first + nunits - 1 of A.F (half_factors
 // != FACT_F32: halves; else floats, split: A.F.split); the multi launch serves
 // items of one (unit size, length kind, penalty, factor kind)

@@ -90,6 +90,7 @@ struct tg_plan {
   // backprojection (plans without the tile-ordered matrix)
   int launch_nb = 1;
   float* d_upd = nullptr;
+  float* d_turned = nullptr;  // IterArgs::turned
   float* d_rep = nullptr;
   float *d_F = nullptr, *d_G = nullptr;
   float* d_stage = nullptr;
@@ -305,6 +306,7 @@ IterArgs make_args(tg_plan* p, int alg, const tg_params* prm) {
   A.slice_id = p->d.slice_id;
   A.num_total_slices = p->d.num_total_slices;
   A.comp = p->d.compensated;
+  A.turned = p->d_turned;
   fill_weights(p, prm, A.pw);
   return A;
 }
@@ -783,6 +785,9 @@ int build_strips(tg_plan* p, const StripTables& T) {
 int ensure_upd(tg_plan* p) {
   if (p->mma) return TG_OK;  // ensure_factors
   if (!p->d_upd) TG_TRY(dalloc(p, &p->d_upd, (size_t)p->R * p->K * p->launch_nb * (p->fp64 ? 2 : 1)));
+  if (p->K == 1 && !p->tiles && !p->fp64 && !p->d_turned && p->S > 1 &&
+      dalloc(p, &p->d_turned, (size_t)p->g2 * p->launch_nb) != TG_OK)
+    p->err.clear();  // the forward projection does without
   if (p->two && !p->d_upd2) TG_TRY(dalloc(p, &p->d_upd2, (size_t)p->R * p->K));
   return TG_OK;
 }
@@ -1212,9 +1217,15 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
   // more slices (1024 x 1024, 720 angles, per 8 slices: 0.96 ms in units of 8,
   // 0.61 of 16, 0.39 of 32), but a small grid has too few blocks to fill the
   // GPU with, so the unit is the largest one that leaves two blocks per SM.
-  // Groups of units (64 slices) are one launch.
+  // Groups of units (64 slices) are one launch. A plan of one to four slices in
+  // one pass keeps the scalar kernels, but on a small grid: there the matrix is
+  // read once all the same, and a unit is mostly padding (MLEM, ms scalar and
+  // tensor: one slice, 256 columns 0.033 and 0.027, 350 columns 0.048 and 0.057,
+  // 709 columns 0.35 and 0.46; four slices, 350 columns 0.059 and 0.057, 709
+  // columns 0.41 and 0.47; SIRT's four 0.62 and 0.54).
   p->mma = d.forward_tiles && !d.backward_staged && !d.compensated &&
-           (d.half_gathers ? M.dlen_kind == LK_F16 : p->K == 8);
+           (d.half_gathers ? M.dlen_kind == LK_F16 : p->K == 8) &&
+           !(d.half_gathers && p->nb == 1 && p->K <= 4 && C >= 320);
   if (p->mma) {
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
