@@ -802,8 +802,8 @@ int build_strips(tg_plan* p, const StripTables& T) {
     int* d_first = nullptr;
     StripExc* d_exc = nullptr;
     if (keep(&d_first, first.size(), false) && keep(&d_exc, (size_t)n, false)) {
-      cudaMemcpy(d_first, first.data(), first.size() * 4, cudaMemcpyHostToDevice);
-      cudaMemcpy(d_exc, e.data(), n * sizeof(StripExc), cudaMemcpyHostToDevice);
+      put(d_first, first.data(), first.size() * 4);
+      put(d_exc, e.data(), n * sizeof(StripExc));
       S.exc_first = d_first;
       S.exc = d_exc;
     } else {
@@ -2095,8 +2095,11 @@ int multi_state(tg_batch* b, const int* algs, const tg_params* params, int it,
   s.key = key;
   s.launches = (int)launches.size();
   cudaError_t e = cudaMalloc(&s.d_items, std::max<size_t>(bytes.size(), 16));
+  // on the stream of the launches: a plain cudaMemcpy from pageable memory may
+  // return before the device has the bytes, and nothing orders it before a
+  // non-blocking stream
   if (e == cudaSuccess)
-    e = cudaMemcpy(s.d_items, bytes.data(), bytes.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(s.d_items, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, b->main);
   cudaGraph_t graph = nullptr;
   if (e == cudaSuccess) e = cudaStreamBeginCapture(b->main, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
