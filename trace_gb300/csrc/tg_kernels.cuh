@@ -467,16 +467,18 @@ void launch_runs_fill(const DevGeom& G, const MatrixDev& M, int tiles_x, int ts,
                       void* tlen, uint32_t* tcode, cudaStream_t st);
 // part: [runs][K] partial sums, written (not accumulated) by each launch;
 // flag, fmax (optional): the batch's non-finite flag and its K slices'
-// largest factors, reset
+// largest factors, reset; width: A.K slices, or the 8 of 8 / A.K batches (half
+// tile, not compensated)
 void launch_forward_tiled(const IterArgs& A, const TileMatrixDev& T,
                           const float* recon_batch, float* part, int* flag, unsigned* fmax,
-                          cudaStream_t st);
+                          int width, cudaStream_t st);
 // ray sums from the partial sums (fixed order) -> per-ray values `out`
 void launch_fwd_finish(const IterArgs& A, const TileMatrixDev& T, const float* part,
                        const float* sino, float* out, int out_mode, cudaStream_t st);
-// the same, factors of slice batch `batch` into A.F
+// the same, factors of the `width` slices from slice batch `batch` on into A.F
 void launch_fwd_finish_units(const IterArgs& A, const TileMatrixDev& T, const float* part,
-                             const float* sino, int batch, int out_mode, cudaStream_t st);
+                             const float* sino, int batch, int out_mode, int width,
+                             cudaStream_t st);
 // units first .. first + nunits - 1 of A.F: floats -> scaled halves (A.F.split)
 void launch_split_factors(const IterArgs& A, int first, int nunits, cudaStream_t st);
 void launch_split_factors_multi(const FinItem* items, int n, int64_t blocks, cudaStream_t st);

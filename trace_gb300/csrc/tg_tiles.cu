@@ -272,6 +272,35 @@ __device__ __forceinline__ void tile_load_half(__half* sm, const float* __restri
   }
 }
 
+// The same for 8 slices from the batches of a plan with sk < 8 slices per pass.
+__device__ __forceinline__ void tile_load_batches(__half* sm, const float* __restrict__ recon,
+                                                  int g, int x0, int y0, int ts, int sk) {
+  const int rs = ts + 1;
+  const int64_t g2 = (int64_t)g * g;
+  for (int e = threadIdx.x; e < ts * ts; e += blockDim.x) {
+    const int ly = e / ts, lx = e - ly * ts;
+    const int x = x0 + lx, y = y0 + ly;
+    Vec<8> v;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v.v[j] = 0.f;
+    if (x < g && y < g) {
+      const int64_t p = (int64_t)y * g + x;
+      if (sk == 4) {
+        const Vec<4> a = load_vec<4>(recon + p * 4), b = load_vec<4>(recon + (g2 + p) * 4);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          v.v[j] = a.v[j];
+          v.v[j + 4] = b.v[j];
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v.v[j] = __ldg(recon + slot_addr(j, p, g2, sk));
+      }
+    }
+    store_hvec<8>(sm + (ly * rs + lx) * 8, v);
+  }
+}
+
 template <int K>
 __device__ __forceinline__ void tile_fma_half(const __half* sm, int si, float l,
                                               float (&acc)[K]) {
@@ -396,10 +425,11 @@ template <int K, int LK, bool H, bool COMP>
 __device__ __forceinline__ void forward_tiled_block(const TileMatrixDev& T, int g,
                                                     float inv_scale, int splits, int block,
                                                     const float* __restrict__ recon,
-                                                    float* __restrict__ part, int* flag, unsigned* fmax) {
+                                                    float* __restrict__ part, int* flag,
+                                                    unsigned* fmax, int sk) {
   extern __shared__ float4 smem4[];
   if (block == 0 && threadIdx.x < K) {
-    if (flag && threadIdx.x == 0) *flag = 0;
+    if (flag && threadIdx.x < K / sk) flag[threadIdx.x] = 0;
     if (fmax) fmax[threadIdx.x] = 0u;
   }
   float* sm = reinterpret_cast<float*>(smem4);
@@ -410,7 +440,9 @@ __device__ __forceinline__ void forward_tiled_block(const TileMatrixDev& T, int 
   const int ts = T.ts, rs = ts + 1;
   const int x0 = (t % T.tiles_x) * ts, y0 = (t / T.tiles_x) * ts;
   const int plane = ts * rs * TilePlanes<K>::kWidth;
-  if constexpr (H)
+  if (K == 8 && H && sk < K)
+    tile_load_batches(smh, recon, g, x0, y0, ts, sk);
+  else if constexpr (H)
     tile_load_half<K>(smh, recon, g, x0, y0, ts);
   else
     tile_load<K>(sm, recon, g, x0, y0, ts);
@@ -476,8 +508,9 @@ template <int K, int LK, bool H, bool COMP>
 __global__ void __launch_bounds__(kBlock)
     k_forward_tiled(TileMatrixDev T, int g, float inv_scale, int splits,
                     const float* __restrict__ recon, float* __restrict__ part, int* flag,
-                    unsigned* fmax) {
-  forward_tiled_block<K, LK, H, COMP>(T, g, inv_scale, splits, blockIdx.x, recon, part, flag, fmax);
+                    unsigned* fmax, int sk) {
+  forward_tiled_block<K, LK, H, COMP>(T, g, inv_scale, splits, blockIdx.x, recon, part, flag,
+                                      fmax, sk);
 }
 
 // Many plans' forward projections in one launch: block -> work item (a
@@ -487,7 +520,7 @@ __global__ void __launch_bounds__(kBlock)
     k_forward_tiled_multi(const FwdItem* __restrict__ items, int nitems) {
   const FwdItem& it = items[item_of(items, nitems, blockIdx.x)];
   forward_tiled_block<K, LK, H, COMP>(it.T, it.g, it.inv_scale, 1,
-                                      (int)(blockIdx.x - it.first), it.recon, it.part, it.flag, it.fmax);
+                                      (int)(blockIdx.x - it.first), it.recon, it.part, it.flag, it.fmax, K);
 }
 
 // A ray's sums: its partial sums (its runs' slots) added in path order.
@@ -518,11 +551,9 @@ __device__ __forceinline__ Vec<K> ray_sums(int64_t r, int n, const int* __restri
 // Ray sums -> per-ray values, as k_forward's epilogue.
 template <int K>
 __device__ __forceinline__ Vec<K> ray_values(int64_t r, const Vec<K>& s,
-                                             const float* __restrict__ ra2,
-                                             const float* __restrict__ sino, int out_mode) {
-  if (out_mode == FWD_SIM) return s;
+                                             const float* __restrict__ ra2, const Vec<K>& ray,
+                                             int out_mode) {
   Vec<K> o;
-  const Vec<K> ray = load_vec<K>(sino + r * K);
   const float a2 = out_mode == FWD_SIRT ? ra2[r] : 1.f;
 #pragma unroll
   for (int j = 0; j < K; ++j)
@@ -541,7 +572,9 @@ __device__ __forceinline__ void fwd_finish_ray(int64_t r, const int* __restrict_
                                                const float* __restrict__ sino,
                                                float* __restrict__ out, int out_mode,
                                                float fofs) {
-  Vec<K> o = ray_values<K>(r, ray_sums<K, COMP>(r, rnrun[r], pbase, part), ra2, sino, out_mode);
+  Vec<K> o = ray_sums<K, COMP>(r, rnrun[r], pbase, part);
+  if (out_mode != FWD_SIM)
+    o = ray_values<K>(r, o, ra2, load_vec<K>(sino + r * K), out_mode);
   if constexpr (FH) {
 #pragma unroll
     for (int j = 0; j < K; ++j) o.v[j] -= fofs;
@@ -553,9 +586,11 @@ __device__ __forceinline__ void fwd_finish_ray(int64_t r, const int* __restrict_
 
 // The same into the units of the tensor-core backprojection (FactorDev).
 // Rays without segments store 0 (no pixel uses them); a non-finite factor
-// raises the batch's flag.
+// raises its batch's flag. sk: slices per pass, 8 / sk batches at K = 8 (R rays
+// between their rows of the sinogram).
 template <int K, bool FH>
-__device__ __forceinline__ void finish_units_ray(int64_t r, const FactorDev& F, int C, int batch,
+__device__ __forceinline__ void finish_units_ray(int64_t r, int64_t R, int sk,
+                                                 const FactorDev& F, int C, int batch,
                                                  const int* __restrict__ rnrun,
                                                  const int* __restrict__ pbase,
                                                  const float* __restrict__ ra2,
@@ -567,22 +602,29 @@ __device__ __forceinline__ void finish_units_ray(int64_t r, const FactorDev& F, 
   for (int j = 0; j < K; ++j) o.v[j] = 0.f;
   const int n = rnrun[r];
   if (n > 0) {
-    o = ray_values<K>(r, ray_sums<K, false>(r, n, pbase, part), ra2, sino, out_mode);
+    Vec<K> ray;
+    if (K == 8 && sk < K) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) ray.v[j] = __ldg(sino + slot_addr(j, r, R, sk));
+    } else {
+      ray = load_vec<K>(sino + r * K);
+    }
+    o = ray_values<K>(r, ray_sums<K, false>(r, n, pbase, part), ra2, ray, out_mode);
     if constexpr (FH) {
 #pragma unroll
       for (int j = 0; j < K; ++j) o.v[j] -= fofs;
     }
   }
   const int a = (int)(r / C), c = (int)(r - (int64_t)a * C);
-  const int unit = batch * K / F.U, su = batch * K % F.U;
+  const int unit = batch * sk / F.U, su = batch * sk % F.U;
   const int64_t e = factor_at((int64_t)(unit % F.ring) * F.unit_elems, F.RP, F.U, a, c, su);
-  bool bad = false;
+  unsigned bad = 0;  // a bit per slice
 #pragma unroll
   for (int j = 0; j < K; ++j) {
     // halves: what rounds to infinity too; floats: the top of the range too,
     // where rounding up to the TF32 part may overflow
-    if constexpr (FH) bad |= !(fabsf(__half2float(__float2half_rn(o.v[j]))) < 7e4f);
-    else bad |= !(fabsf(o.v[j]) < 1e38f);
+    if constexpr (FH) bad |= !(fabsf(__half2float(__float2half_rn(o.v[j]))) < 7e4f) ? 1u << j : 0u;
+    else bad |= !(fabsf(o.v[j]) < 1e38f) ? 1u << j : 0u;
   }
   if constexpr (FH) {
     store_hvec<K>(reinterpret_cast<__half*>(F.base) + e, o);
@@ -593,12 +635,13 @@ __device__ __forceinline__ void finish_units_ray(int64_t r, const FactorDev& F, 
       for (int j = 0; j < K; ++j) {
         const unsigned act = __activemask();
         const unsigned m = __reduce_max_sync(act, __float_as_uint(fabsf(o.v[j])));
-        if ((threadIdx.x & 31) == __ffs(act) - 1 && m > F.fmax[batch * K + j])
-          atomicMax(F.fmax + batch * K + j, m);
+        if ((threadIdx.x & 31) == __ffs(act) - 1 && m > F.fmax[batch * sk + j])
+          atomicMax(F.fmax + batch * sk + j, m);
       }
     }
   }
-  if (bad) F.flags[batch] = 1;
+  for (int b = 0; bad; ++b, bad >>= sk)
+    if (bad & ((1u << sk) - 1u)) F.flags[batch + b] = 1;
 }
 
 // Float factors of one column and 8 slices -> high and low halves (FactorDev).
@@ -639,13 +682,14 @@ __global__ void k_split_factors_multi(const FinItem* __restrict__ items, int nit
 
 template <int K, bool FH>
 __global__ void k_fwd_finish_units(int64_t nrays, const __grid_constant__ FactorDev F, int C,
-                                   int batch, const int* __restrict__ rnrun,
+                                   int batch, int sk, const int* __restrict__ rnrun,
                                    const int* __restrict__ pbase, const float* __restrict__ ra2,
                                    const float* __restrict__ part,
                                    const float* __restrict__ sino, int out_mode, float fofs) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r < nrays)
-    finish_units_ray<K, FH>(r, F, C, batch, rnrun, pbase, ra2, part, sino, out_mode, fofs);
+    finish_units_ray<K, FH>(r, nrays, sk, F, C, batch, rnrun, pbase, ra2, part, sino, out_mode,
+                            fofs);
 }
 
 template <int K, bool FH, bool COMP>
@@ -668,10 +712,10 @@ __global__ void k_fwd_finish_multi(const FinItem* __restrict__ items, int nitems
   if (r >= it.nrays) return;
   if (!COMP && it.F.U) {
     if (it.fh != FACT_F32)
-      finish_units_ray<K, true>(r, it.F, it.C, it.batch, it.rnrun, it.pbase, it.ra2,
+      finish_units_ray<K, true>(r, it.nrays, K, it.F, it.C, it.batch, it.rnrun, it.pbase, it.ra2,
                                 it.part, it.sino, it.out_mode, factor_offset(it.fh));
     else
-      finish_units_ray<K, false>(r, it.F, it.C, it.batch, it.rnrun, it.pbase, it.ra2,
+      finish_units_ray<K, false>(r, it.nrays, K, it.F, it.C, it.batch, it.rnrun, it.pbase, it.ra2,
                                  it.part, it.sino, it.out_mode, 0.f);
     return;
   }
@@ -685,7 +729,8 @@ __global__ void k_fwd_finish_multi(const FinItem* __restrict__ items, int nitems
 
 template <int K, int LK, bool H, bool COMP>
 void fwd_tiled_launch(const TileMatrixDev& T, int g, float inv_scale,
-                      const float* recon, float* part, int* flag, unsigned* fmax, cudaStream_t st) {
+                      const float* recon, float* part, int* flag, unsigned* fmax, int sk,
+                      cudaStream_t st) {
   const int smem = TilePlanes<K, H>::bytes(T.ts);
   cudaFuncSetAttribute(k_forward_tiled<K, LK, H, COMP>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -695,18 +740,22 @@ void fwd_tiled_launch(const TileMatrixDev& T, int g, float inv_scale,
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int splits = max(1, min(16, (2 * sms + T.ntiles - 1) / T.ntiles));
   k_forward_tiled<K, LK, H, COMP><<<T.ntiles * splits, T.bw * 32, smem, st>>>(
-      T, g, inv_scale, splits, recon, part, flag, fmax);
+      T, g, inv_scale, splits, recon, part, flag, fmax, sk);
 }
 
 template <int K, bool H, bool COMP>
 void fwd_tiled_kind(const TileMatrixDev& T, int g, int len_kind, float inv_scale,
-                    const float* recon, float* part, int* flag, unsigned* fmax, cudaStream_t st) {
+                    const float* recon, float* part, int* flag, unsigned* fmax, int sk,
+                    cudaStream_t st) {
+#define TG_TILED(LKK) \
+  fwd_tiled_launch<K, LKK, H, COMP>(T, g, inv_scale, recon, part, flag, fmax, sk, st)
   switch (len_kind) {
-    case LK_F32: fwd_tiled_launch<K, LK_F32, H, COMP>(T, g, inv_scale, recon, part, flag, fmax, st); break;
-    case LK_BF16: fwd_tiled_launch<K, LK_BF16, H, COMP>(T, g, inv_scale, recon, part, flag, fmax, st); break;
-    case LK_F16: fwd_tiled_launch<K, LK_F16, H, COMP>(T, g, inv_scale, recon, part, flag, fmax, st); break;
-    default: fwd_tiled_launch<K, LK_U16, H, COMP>(T, g, inv_scale, recon, part, flag, fmax, st); break;
+    case LK_F32: TG_TILED(LK_F32); break;
+    case LK_BF16: TG_TILED(LK_BF16); break;
+    case LK_F16: TG_TILED(LK_F16); break;
+    default: TG_TILED(LK_U16); break;
   }
+#undef TG_TILED
 }
 
 template <int K, bool COMP>
@@ -715,9 +764,11 @@ void fwd_tiled_half(const IterArgs& A, const TileMatrixDev& T, const float* reco
   // an f32 tile of 16 slices would not fit shared memory (plan creation
   // requires half_gathers with 16 slices per pass and forward_tiles)
   if (K == 16 || A.half_tile)
-    fwd_tiled_kind<K, true, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, flag, fmax, st);
+    fwd_tiled_kind<K, true, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, flag, fmax,
+                                  A.K, st);
   else if constexpr (K != 16)
-    fwd_tiled_kind<K, false, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, flag, fmax, st);
+    fwd_tiled_kind<K, false, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, flag, fmax,
+                                   A.K, st);
 }
 
 // compensated sums: up to 8 slices per pass (plan creation checks)
@@ -854,8 +905,9 @@ void launch_runs_fill(const DevGeom& G, const MatrixDev& M, int tiles_x, int ts,
 }
 
 void launch_forward_tiled(const IterArgs& A, const TileMatrixDev& T,
-                          const float* recon_batch, float* part, int* flag, unsigned* fmax, cudaStream_t st) {
-  switch (A.K) {
+                          const float* recon_batch, float* part, int* flag, unsigned* fmax,
+                          int width, cudaStream_t st) {
+  switch (width) {
     case 1: fwd_tiled_comp<1>(A, T, recon_batch, part, flag, fmax, st); break;
     case 2: fwd_tiled_comp<2>(A, T, recon_batch, part, flag, fmax, st); break;
     case 4: fwd_tiled_comp<4>(A, T, recon_batch, part, flag, fmax, st); break;
@@ -899,17 +951,18 @@ static void finish_units_k(const IterArgs& A, const TileMatrixDev& T, const floa
   const int64_t R = (int64_t)A.G.P * A.G.C;
   const int b = blocks_for(R, 256);
   if (A.half_factors != FACT_F32)
-    k_fwd_finish_units<K, true><<<b, 256, 0, st>>>(R, A.F, A.G.C, batch, T.rnrun, T.pbase,
+    k_fwd_finish_units<K, true><<<b, 256, 0, st>>>(R, A.F, A.G.C, batch, A.K, T.rnrun, T.pbase,
                                                    A.M.ra2, part, sino, out_mode,
                                                    factor_offset(A.half_factors));
   else
-    k_fwd_finish_units<K, false><<<b, 256, 0, st>>>(R, A.F, A.G.C, batch, T.rnrun, T.pbase,
+    k_fwd_finish_units<K, false><<<b, 256, 0, st>>>(R, A.F, A.G.C, batch, A.K, T.rnrun, T.pbase,
                                                     A.M.ra2, part, sino, out_mode, 0.f);
 }
 
 void launch_fwd_finish_units(const IterArgs& A, const TileMatrixDev& T, const float* part,
-                             const float* sino, int batch, int out_mode, cudaStream_t st) {
-  switch (A.K) {
+                             const float* sino, int batch, int out_mode, int width,
+                             cudaStream_t st) {
+  switch (width) {
     case 1: finish_units_k<1>(A, T, part, sino, batch, out_mode, st); break;
     case 2: finish_units_k<2>(A, T, part, sino, batch, out_mode, st); break;
     case 4: finish_units_k<4>(A, T, part, sino, batch, out_mode, st); break;
