@@ -373,9 +373,22 @@ void drop_graphs(tg_plan* p) {
   }
 }
 
+// Whether captured iterations are worth two branches, and outlive a reset of the
+// reconstruction whose buffers stay. A graph of two branches takes the host some
+// 60 us to launch, and destroying a graph that still runs waits for it. For long
+// iterations the branches fill each other's tails and the wait is what costs
+// (725 columns, 411 angles, 13 slices, 2 MLEM iterations: 1.83 ms a pass among
+// others and 1.95 alone; 1.97 and 1.98 captured anew each pass; 1.83 and 2.14 on
+// one branch). For short ones the launch costs more than it hides (67 columns,
+// 45 angles, 14 slices, 3 APMLR iterations: 107 us on one branch, 208 on two),
+// and the wait keeps the host from filling the GPU's launch queue (128 columns,
+// one slice, 10 iterations, 3000 passes ahead: 140 us a pass, 690 without).
+// The line is about 0.25 ms an iteration.
+bool long_pass(const tg_plan* p) { return p->g2 * p->P * p->S >= 500000000; }
+
 int establish_layout(tg_plan* p, int alg) {
   if (!valid_alg(alg)) return fail(p, TG_E_ARG, "unknown algorithm");
-  drop_graphs(p);
+  if (!long_pass(p)) drop_graphs(p);
   const int halo = halo_of(alg);
   int vshift = 0, fshift = 0;
   if (alg == TG_APMLR) {
@@ -391,6 +404,7 @@ int establish_layout(tg_plan* p, int alg) {
   const int nslots = (need + p->K - 1) / p->K * p->K;
   if (p->layout_alg < 0 || p->nslots != nslots || p->halo != halo ||
       p->vshift != vshift) {
+    drop_graphs(p);  // captured iterations hold the buffers' addresses
     const size_t esz = p->fp64 ? 2 : 1;  // floats per element
     const size_t old_n = (size_t)p->nslots * p->g2 * esz;
     for (int b = 0; b < 2; ++b) {
@@ -1773,7 +1787,7 @@ int tg_iterate(tg_plan* p, int alg, const tg_params* prm, int n_iter) {
         g = tg_plan::Graph();
         cudaGraph_t graph;
         TG_CUDA(p, cudaStreamBeginCapture(p->st, cudaStreamCaptureModeThreadLocal));
-        issue_iteration(p, A, mode, true);
+        issue_iteration(p, A, mode, long_pass(p));
         TG_CUDA(p, cudaStreamEndCapture(p->st, &graph));
         const cudaError_t e = cudaGraphInstantiate(&g.exec, graph, 0);
         cudaGraphDestroy(graph);
