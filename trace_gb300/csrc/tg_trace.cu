@@ -84,7 +84,11 @@ __global__ void __launch_bounds__(kTraceBlock)
   // A ray's first visit of a pixel stores its length without reading the slot,
   // which no other ray has: a pixel further along the path in x or in y than
   // all before it is new. The read cost a wait per segment (256 columns, 180
-  // angles: 524 us, 406 without; 1024 columns, 720 angles: 8.7 ms, 7.6).
+  // angles: 524 us, 406 without; 1024 columns, 720 angles: 8.7 ms, 7.6). Four
+  // angles share 16 bytes of a pixel, which then wait in L2 for the next angle:
+  // where a grid's do not fit, the stores go out as partial sectors and the read
+  // is the cheaper way (2048 columns, 1500 angles: 64 ms, 72 without).
+  const bool fits = (int64_t)G.C * G.C * 16 <= (32 << 20);
   const int ydir = G.quad[a] ? 1 : -1;
   int most_x = INT_MIN, most_y = INT_MIN;
   trace_ray(G, a, c, [&](int idx, float l, float l2, int ix, int iy) {
@@ -134,7 +138,7 @@ __global__ void __launch_bounds__(kTraceBlock)
       int tile, tl;
       pixel_tile(ix, iy, M.tiles_x, M.tw_shift, &tile, &tl);
       const int64_t pos = dense_pair(M.ntiles, a, tile, tl) * 2 + slot;
-      const bool first = ix > most_x || iy * ydir > most_y;
+      const bool first = fits && (ix > most_x || iy * ydir > most_y);
       if (L16) {
         uint16_t* d = reinterpret_cast<uint16_t*>(dlen);
         const float cur = first ? 0.f : decode16(d[pos], M.dlen_kind, M.inv_scale);
