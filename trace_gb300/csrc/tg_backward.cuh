@@ -209,10 +209,11 @@ constexpr int min_blocks() {
 
 // COMP: compensated summation - each quad's (four angles') products are an
 // FMA chain added to the pixel's sum with Kahan's correction.
-// One block's work (8 pixel tiles, from tile block * kWarps);
+// One block's work (8 pixel tiles, from tile block * kWarps) for batch `batch`,
+// its factors ub batches behind upd;
 // s_coef: the block's kCoefChunk-entry shared buffer of window coefficients.
 template <int K, int LK, bool EXACT, bool PEN, bool FH, bool COMP>
-__device__ __forceinline__ void backward_block(const IterArgs& A, int batch, int block,
+__device__ __forceinline__ void backward_block(const IterArgs& A, int batch, int ub, int block,
                                                const float* __restrict__ cur,
                                                float* __restrict__ next,
                                                const float* __restrict__ upd,
@@ -251,7 +252,8 @@ __device__ __forceinline__ void backward_block(const IterArgs& A, int batch, int
   const uint32_t qstep = (uint32_t)A.M.ntiles * 32 * QW;  // words per 4 angles
   const uint4* qp = reinterpret_cast<const uint4*>(A.M.dlen) + ((int64_t)tile * 32 + lane) * QW;
   const int ck = G.C * K;  // factor floats per angle
-  const float* ua = upd;
+  const int64_t per_batch = (int64_t)G.P * ck;
+  const float* ua = FH ? upd : upd + ub * per_batch;
   for (int a0 = 0; a0 < P4; a0 += kCoefChunk) {
     const int na = min(kCoefChunk, P4 - a0);  // a multiple of 4
     __syncthreads();
@@ -356,7 +358,11 @@ __device__ __forceinline__ void backward_block(const IterArgs& A, int batch, int
   }
   // segments outside the pixel's window (stored apart, true lengths)
   for_each_exception(A.M, tile, lane, [&](float l, int ea, int ec) {
-    const int64_t e = ((int64_t)ea * G.C + ec) * K;
+    // the batch's factors found anew: kept, they would cost the angle loop two
+    // registers (and it spills)
+    int b = ub;
+    asm volatile("" : "+r"(b));
+    const int64_t e = (FH ? 0 : b * ((int64_t)G.P * G.C * K)) + ((int64_t)ea * G.C + ec) * K;
     const float* ub = FH ? reinterpret_cast<const float*>(
                                reinterpret_cast<const __half*>(upd) + e)
                          : upd + e;
@@ -392,9 +398,8 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<K, COMP>()))
   // a piece of the matrix while it is in L2
   // (tile-staged plans, which half factors imply, launch one batch)
   const int b = FH ? 0 : blockIdx.x;
-  const float* u = FH ? upd : upd + b * ((int64_t)A.G.P * A.G.C * K);
-  backward_block<K, LK, EXACT, PEN, FH, COMP>(A, first + b, grid_block(), cur, next, u, rep_num, epi,
-                                              s_coef);
+  backward_block<K, LK, EXACT, PEN, FH, COMP>(A, first + b, b, grid_block(), cur, next, upd,
+                                              rep_num, epi, s_coef);
 }
 
 // Many plans' fused backprojection + update in one launch (fast mode):
@@ -404,7 +409,7 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<K, COMP>()))
     k_backward_multi(const BackItem* __restrict__ items, int nitems) {
   __shared__ float4 s_coef[kCoefChunk];
   const BackItem& it = items[item_of(items, nitems, blockIdx.x)];
-  backward_block<K, LK, false, PEN, FH, COMP>(it.A, it.batch, (int)(blockIdx.x - it.first),
+  backward_block<K, LK, false, PEN, FH, COMP>(it.A, it.batch, 0, (int)(blockIdx.x - it.first),
                                               it.cur, it.next, it.upd, nullptr, EPI_UPDATE,
                                               s_coef);
 }

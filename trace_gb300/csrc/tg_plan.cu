@@ -383,7 +383,8 @@ void drop_graphs(tg_plan* p) {
 // 45 angles, 14 slices, 3 APMLR iterations: 107 us on one branch, 208 on two),
 // and the wait keeps the host from filling the GPU's launch queue (128 columns,
 // one slice, 10 iterations, 3000 passes ahead: 140 us a pass, 690 without).
-// The line is about 0.25 ms an iteration.
+// The line is about 0.25 ms an iteration. (The scalar kernels' two chains have
+// nothing to wait for but their end: two branches always.)
 bool long_pass(const tg_plan* p) { return p->g2 * p->P * p->S >= 500000000; }
 
 int establish_layout(tg_plan* p, int alg) {
@@ -749,6 +750,15 @@ int build_strips(tg_plan* p, const StripTables& T) {
   uint8_t* grazed;
   const size_t nsteps = (size_t)S.nbundles * (T.R / 4);
   const size_t U = std::min(p->group_units * p->unit, p->S) <= 32 ? 32 : 64;
+  size_t free_bytes = 0, total_bytes = 0;
+  if (cudaMemGetInfo(&free_bytes, &total_bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return TG_OK;
+  }
+  if (nsteps * (64 * sizeof(*codes) + 16 * sizeof(*meta)) +
+          U * (p->g2 * sizeof(*p->d_simg) + S.nbundles * 16 * sizeof(*p->d_spart)) >
+      free_bytes / 2)
+    return TG_OK;
   StripExc* exc = nullptr;
   int* nexc = nullptr;
   constexpr int kCap = 1 << 20;
@@ -1273,7 +1283,9 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
   (void)counters[1];
   // The backprojection runs on the tensor cores for half-gather plans with
   // 16-bit lengths (f16 in the backward matrix), and for FP32 operands at 8
-  // slices per pass. A larger unit of slices spreads a tile's A operand over
+  // slices per pass or where a unit serves several passes (768 x 768, 540 angles,
+  // 16 slices, 2 PML iterations: 8 per pass 6.8 ms scalar and 5.6, 4 per pass 7.9
+  // and 6.2). A larger unit of slices spreads a tile's A operand over
   // more slices (1024 x 1024, 720 angles, per 8 slices: 0.96 ms in units of 8,
   // 0.61 of 16, 0.39 of 32), but a small grid has too few blocks to fill the
   // GPU with, so the unit is the largest one that leaves two blocks per SM.
@@ -1284,14 +1296,17 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
   // 709 columns 0.35 and 0.46; four slices, 350 columns 0.059 and 0.057, 709
   // columns 0.41 and 0.47; SIRT's four 0.62 and 0.54).
   p->mma = d.forward_tiles && !d.backward_staged && !d.compensated &&
-           (d.half_gathers ? M.dlen_kind == LK_F16 : p->K == 8) &&
+           (d.half_gathers ? M.dlen_kind == LK_F16 : p->K <= 8) &&
            !(d.half_gathers && p->nb == 1 && p->K <= 4 && C >= 320);
+  int U = p->S <= 8 ? 8 : p->S <= 16 ? 16 : 32;
   if (p->mma) {
     int sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int U = p->S <= 8 ? 8 : p->S <= 16 ? 16 : 32;
     while (U > 8 && mma_regions(C) * ((p->S + U - 1) / U) < 2 * sms) U /= 2;
+    if (!d.half_gathers && p->K < 8) p->mma = U > p->K && p->S > 4;
+  }
+  if (p->mma) {
     p->unit = std::max(U, p->K);
     p->nunits = (p->S + p->unit - 1) / p->unit;
     p->group_units = std::min(std::max(1, 64 / p->unit), p->nunits);
@@ -1312,7 +1327,8 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
   // slices. 1024 x 1024 x 720, forward and finish: 32 slices 4.1 ms in tiles,
   // 2.9 in strips; 64 slices 8.2 and 4.6; 24 slices 3.1 and 2.9, which is not
   // worth the memory. A plan that traces on the fly, to save memory, keeps the
-  // tiles too.
+  // tiles too, and so does one whose strips would take more than half of the free
+  // memory, which may be meant for other plans.
   if (p->mma && d.half_gathers && p->len_kind == TG_LEN_U16 && !otf && p->S >= 32) {
     StripTables T;
     T.entries = entries;
@@ -1787,7 +1803,7 @@ int tg_iterate(tg_plan* p, int alg, const tg_params* prm, int n_iter) {
         g = tg_plan::Graph();
         cudaGraph_t graph;
         TG_CUDA(p, cudaStreamBeginCapture(p->st, cudaStreamCaptureModeThreadLocal));
-        issue_iteration(p, A, mode, long_pass(p));
+        issue_iteration(p, A, mode, !p->mma || long_pass(p));
         TG_CUDA(p, cudaStreamEndCapture(p->st, &graph));
         const cudaError_t e = cudaGraphInstantiate(&g.exec, graph, 0);
         cudaGraphDestroy(graph);
