@@ -402,6 +402,16 @@ def format_bytes(info, W, K, tiles, half=False):
     return fwd, back
 
 
+def kernel_names(info, args, W, K, nb, per_step):
+    """The forward and the backward kernel of the schedule that was timed."""
+    if not args.tiles:
+        return "k_forward", "k_backward"
+    strips = info["tile_runs"] % (W["P"] * W["C"]) == 0 and per_step["forward"] < nb
+    mma = per_step["backward"] < nb or (not args.staged and not args.compensated and K >= 8)
+    return ("k_forward_strips" if strips else "k_forward_tiled",
+            "k_backward_mma" if mma else "k_backward")
+
+
 def run_ours(args, W):
     import numpy as np
     import torch
@@ -481,22 +491,36 @@ def _run_ours(args, W, ws, rank, local, dev, stream, tg, torch, np):
     # per-kernel device times from a separate pass after the timed region
     # (the per-launch timers run eagerly, outside any graph)
     plan.set_timing(True)
-    time_iterations(plan, alg, prm, max(2, min(args.steps, 3)), stream, torch)
+    timed = max(2, min(args.steps, 3))
+    time_iterations(plan, alg, prm, timed, stream, torch)
     tim = plan.timing()
     plan.set_timing(False)
     ms_max = max_over_ranks(ms, ws)
     slice_iters = S * args.steps * ws
     value = slice_iters / (ms_max / 1000.0)
     nb = info["batches"]
-    launches = args.steps * nb * (3 if args.tiles else 2)
 
-    fwd_b, back_b = kernel_bytes(info, W, K, args.len_storage)
-    fwd_f, back_f = format_bytes(info, W, K, args.tiles, args.half)
+    # a launch serves one slice batch or, on the tensor cores, several of them:
+    # its bytes are those of one matrix pass for all of its slices
+    per_step = {k: max(tim[k + "_launches"] / timed, 1) for k in ("forward", "backward", "other")}
+    slices = {k: min(nb * K / n, S) for k, n in per_step.items()}
+    fwd_b = kernel_bytes(info, W, slices["forward"], args.len_storage)[0]
+    back_b = kernel_bytes(info, W, slices["backward"], args.len_storage)[1]
+    fwd_f = format_bytes(info, W, slices["forward"], args.tiles, args.half)[0]
+    back_f = format_bytes(info, W, slices["backward"], args.tiles, args.half)[1]
     fwd_avg = tim["forward_ms"] / max(tim["forward_launches"], 1)
     back_avg = tim["backward_ms"] / max(tim["backward_launches"], 1)
     dom = "backward" if tim["backward_ms"] >= tim["forward_ms"] else "forward"
-    kname = {"forward": "k_forward_tiled" if args.tiles else "k_forward",
-             "backward": "k_backward"}[dom]
+    kf, kb = kernel_names(info, args, W, K, nb, per_step)
+    kname = {"forward": kf, "backward": kb}[dom]
+    # the strips' forward is three launches (reset, halves, sums), the tensor-core
+    # backprojection of SIRT's float factors two (their halves first)
+    launches = round(args.steps * (sum(per_step.values()) if args.tiles
+                                   else per_step["forward"] + per_step["backward"]))
+    if kf == "k_forward_strips":
+        launches += round(2 * args.steps * per_step["forward"])
+    if kb == "k_backward_mma" and args.half and alg == "sirt":
+        launches += round(args.steps * per_step["backward"])
     dom_bytes, dom_ms = (back_b, back_avg) if dom == "backward" else (fwd_b, fwd_avg)
     achieved = dom_bytes / (dom_ms / 1000.0) / 1e9
     traffic = ncu_traffic().get(f"{kname}:{args.workload}:{args.len_storage}:K{K}"
@@ -519,14 +543,16 @@ def _run_ours(args, W, ws, rank, local, dev, stream, tg, torch, np):
         "share": (tim["backward_ms"] if dom == "backward" else tim["forward_ms"]) /
                  max(tim["forward_ms"] + tim["backward_ms"], 1e-9),
         "kernels": {
-            ("k_forward_tiled" if args.tiles else "k_forward"): {
+            kf: {
                 "avg_ms": fwd_avg, "bytes": fwd_b, "gbs": gbs(fwd_b, fwd_avg),
                 "format_bytes": fwd_f, "format_gbs": gbs(fwd_f, fwd_avg)},
-            "k_fwd_finish": {"avg_ms": tim["other_ms"] / max(tim["other_launches"], 1),
-                             "format_bytes": 4 * info["partial_slots"] * K
-                                             + 4 * W["P"] * W["C"] * K * 2},
-            "k_backward": {"avg_ms": back_avg, "bytes": back_b, "gbs": gbs(back_b, back_avg),
-                           "format_bytes": back_f, "format_gbs": gbs(back_f, back_avg)},
+            "k_strips_finish" if kf == "k_forward_strips" else "k_fwd_finish": {
+                "avg_ms": tim["other_ms"] / max(tim["other_launches"], 1),
+                "format_bytes": (4 * info["partial_slots"]
+                                 + 4 * W["P"] * W["C"] * 2) * slices["other"]},
+            kb: {
+                "avg_ms": back_avg, "bytes": back_b, "gbs": gbs(back_b, back_avg),
+                "format_bytes": back_f, "format_gbs": gbs(back_f, back_avg)},
         },
     }
 
@@ -573,7 +599,9 @@ def _run_ours(args, W, ws, rank, local, dev, stream, tg, torch, np):
                    "len_storage": args.len_storage, "index": "4-bit delta",
                    "gather_operands": "f16 (tile, factor-1)" if args.half else "f32",
                    "intersections": "traced on the fly" if args.otf else "cached",
-                   "forward": (f"tile-staged ({args.fts or 64}x{args.fts or 64} "
+                   "forward": "strip-ordered (16-ray bundles, tensor cores)"
+                              if kf == "k_forward_strips" else
+                              (f"tile-staged ({args.fts or 64}x{args.fts or 64} "
                                "shared-memory tiles)") if args.tiles else "ray-ordered",
                    "backward_tile": {4: "4x8", 16: "16x2"}.get(args.btw, "8x4") + " pixels",
                    "forward_block_warps": args.fbw or 32,
