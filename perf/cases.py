@@ -122,7 +122,7 @@ def _problems(c):
     for i in range(c["count"]):
         C = r.choice([c["C"] // 4, c["C"] // 2, c["C"] * 3 // 4, c["C"]])
         out.append(dict(c, kind="iterate", alg="sirt" if i % 2 == 0 else "mlem", C=C,
-                        P=r.randint(90, c["P"]), S=r.randint(1, c["S"])))
+                        P=r.randint(min(90, c["P"]), c["P"]), S=r.randint(1, c["S"])))
     return out
 
 
