@@ -1888,12 +1888,10 @@ struct tg_batch {
   cudaStream_t main = nullptr;
   cudaEvent_t fork = nullptr;
   std::vector<cudaEvent_t> joins;
+  // plans that the multi-plan launches do not take: one captured iteration per
+  // parity of plan 0's buffers, valid for one multi_key
   struct Graph {
-    bool valid = false;
-    std::vector<int> algs;
-    std::vector<int> half_factors;  // per plan, as issue_iteration decides
-    std::vector<tg_params> prms;
-    int cur0 = -1;  // plan 0's buffer parity the graph was captured in
+    std::string key;
     cudaGraphExec_t exec = nullptr;
   } graphs[2];
   std::string err;
@@ -2294,16 +2292,11 @@ extern "C" int tg_batch_iterate(tg_batch* b, const int* algs, const tg_params* p
                                : p->nb * (p->tiles ? 3 : 2);
   }
   for (int it = 0; it < n_iter; ++it) {
-    const int parity = b->plans[0]->cur;
-    tg_batch::Graph& g = b->graphs[parity];
-    std::vector<int> hf(n);
-    for (int i = 0; i < n; ++i)
-      hf[i] = half_factors_next(b->plans[i], algs[i] == TG_SIRT ? FWD_SIRT : FWD_RATIO);
-    bool match = g.valid && g.cur0 == parity && g.half_factors == hf;
-    for (int i = 0; match && i < n; ++i)
-      match = g.algs[i] == algs[i] &&
-              same_params(g.prms[i], params ? &params[i] : nullptr);
-    if (!match) {
+    // the key holds every plan's parity and buffers: a plan may have been reset,
+    // or given another layout, by itself since the capture
+    tg_batch::Graph& g = b->graphs[b->plans[0]->cur];
+    const std::string key = multi_key(b, algs, params, 0);
+    if (!g.exec || g.key != key) {
       if (g.exec) cudaGraphExecDestroy(g.exec);
       g = tg_batch::Graph();
       cudaGraph_t graph;
@@ -2334,11 +2327,7 @@ extern "C" int tg_batch_iterate(tg_batch* b, const int* algs, const tg_params* p
         b->err = std::string("graph capture failed: ") + cudaGetErrorString(e);
         return TG_E_CUDA;
       }
-      g.valid = true;
-      g.cur0 = parity;
-      g.half_factors = hf;
-      g.algs.assign(algs, algs + n);
-      for (int i = 0; i < n; ++i) g.prms.push_back(params ? params[i] : tg_params{});
+      g.key = key;
     }
     const cudaError_t e = cudaGraphLaunch(g.exec, b->main);
     if (e != cudaSuccess) {
