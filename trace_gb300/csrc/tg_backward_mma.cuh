@@ -49,9 +49,10 @@
 // are split too, the two low parts' product left out.
 //
 // A zero of A times a non-finite factor would reach pixels that the ray does
-// not cross: the finish kernel raises the batch's flag when it stores a
-// non-finite factor for a ray with segments, and the kernel then sums per
-// crossed ray (slow_sum), as the scalar kernel does.
+// not cross: the finish kernel marks the slice when it stores a non-finite
+// factor for a ray with segments, and the kernel then takes that slice's sums
+// per crossed ray (slow_sum), as the scalar kernel does. The columns of a
+// product are independent, so the other slices' stay.
 //
 // Measured (1024 x 1024, 720 angles, ms per 8 slices; the scalar kernel of
 // tg_backward.cuh before the arrow): MLEM half factors 1.15 -> 0.96 in units
@@ -193,33 +194,56 @@ __device__ __forceinline__ void pair_lengths(const PairWord<LK>& w, float& l0, f
   }
 }
 
-// Sum over the pixel's crossed rays of one slice, one product at a time (the
-// path taken when a factor is not finite): `at` is the pixel's first pair.
+// Sum over the pixel's crossed rays of one slice, one product at a time, of
+// every other angle quad from q0 on (the path taken when a factor is not
+// finite): `at` is the pixel's first pair. The four angles' factors are in
+// flight together.
 template <int LK, bool HALF>
-__device__ __noinline__ float slow_sum(const IterArgs& A, const uint32_t* at, int x, int y,
+__device__ __noinline__ float slow_sum(const IterArgs& A, const uint32_t* at, int x, int y, int q0,
                                        int64_t unit_base, int su) {
   constexpr int W = LK == LK_F32 ? 2 : 1;
   const int U = A.F.U, RP = A.F.RP;
   float acc = 0.f;
-  for (int a = 0; a < A.G.P; ++a) {
-    const uint32_t* q = at + ((int64_t)(a >> 2) * A.M.ntiles * 128 + (a & 3)) * W;
-    PairWord<LK> w;
-    for (int k = 0; k < W; ++k) w.v[k] = q[k];
-    const bool h0 = LK == LK_F32 ? w.v[0] != 0u : (w.v[0] & 0xffffu) != 0u;
-    const bool h1 = LK == LK_F32 ? w.v[W - 1] != 0u : (w.v[0] >> 16) != 0u;
-    if (!(h0 | h1)) continue;
-    float l[2];
-    pair_lengths<LK>(w, l[0], l[1]);
-    const int c0 = window_c0(A.M.wcoef[a], (float)x, (float)y);
-    for (int k = 0; k < 2; ++k) {
-      if (!(k ? h1 : h0)) continue;
-      const int64_t e = factor_at(unit_base, RP, U, a, c0 + k, su);
-      const float f = HALF ? __half2float(reinterpret_cast<const __half*>(A.F.base)[e])
-                           : reinterpret_cast<const float*>(A.F.base)[e];
-      acc = fmaf(l[k], f, acc);
+  for (int q = q0; q < A.M.P4 / 4; q += 2) {
+    const uint4* w = reinterpret_cast<const uint4*>(at + (int64_t)q * A.M.ntiles * (128 * W));
+    uint32_t v[4 * W];
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      const uint4 t = __ldg(w + k);
+      v[4 * k] = t.x; v[4 * k + 1] = t.y; v[4 * k + 2] = t.z; v[4 * k + 3] = t.w;
     }
+    float l[8], f[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      PairWord<LK> p;
+#pragma unroll
+      for (int k = 0; k < W; ++k) p.v[k] = v[j * W + k];
+      const bool h0 = LK == LK_F32 ? p.v[0] != 0u : (p.v[0] & 0xffffu) != 0u;
+      const bool h1 = LK == LK_F32 ? p.v[W - 1] != 0u : (p.v[0] >> 16) != 0u;
+      pair_lengths<LK>(p, l[2 * j], l[2 * j + 1]);
+      const int a = q * 4 + j, c0 = window_c0(__ldg(A.M.wcoef + a), (float)x, (float)y);
+      const int64_t e = factor_at(unit_base, RP, U, a, c0, su);
+      f[2 * j] = f[2 * j + 1] = 0.f;
+      if constexpr (HALF) {
+        const __half* b = reinterpret_cast<const __half*>(A.F.base) + e;
+        if (h0) f[2 * j] = __half2float(b[0]);
+        if (h1) f[2 * j + 1] = __half2float(b[U]);
+      } else {
+        const float* b = reinterpret_cast<const float*>(A.F.base) + e;
+        if (h0) f[2 * j] = b[0];
+        if (h1) f[2 * j + 1] = b[U];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc = fmaf(l[i], f[i], acc);
   }
   return acc;
+}
+
+// A bit per slice of the unit: those with a non-finite factor.
+__device__ __forceinline__ unsigned bad_slices(const IterArgs& A, int unit, int lane) {
+  const int s = unit * A.F.U + lane;
+  return __ballot_sync(0xffffffffu, lane < A.F.U && s < A.S && A.F.stat[s].bad != 0);
 }
 
 // n <= N consecutive slots' values of one pixel, slot s's at `r` (one vector
@@ -341,11 +365,7 @@ __device__ __forceinline__ void backward_mma_block(const IterArgs& A, int unit, 
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[j][i] = 0.f;
 
-  bool finite = true;
-  for (int b = unit * U / A.K; b < A.F.nflags && b * A.K < (unit + 1) * U; ++b)
-    finite &= A.F.flags[b] == 0;
-
-  if (finite) {
+  {
     // length pairs: the thread copies one pixel (rows of 16 pixels, the
     // matrix's order), of every other angle quad
     const int cx = X0 + (tid & 15), cy = Y0 + ((tid >> 4) & 7);
@@ -576,6 +596,31 @@ __device__ __forceinline__ void backward_mma_block(const IterArgs& A, int unit, 
     }
   }
 
+  // Slices with a non-finite factor: their sums again, ray by ray, into shared
+  // memory ([warp][16 pixels][U]; kept out of the accumulators' registers). A lane
+  // takes one of the tile's 16 pixels and half of the angle quads.
+  const unsigned bad = bad_slices(A, unit, lane);
+  float* const again = reinterpret_cast<float*>(sm) + warp * 16 * U;
+  static_assert(kMmaTiles * 16 * U * 4 <= St::kBytes, "the sums fit the stages");
+  if (bad) {
+    __syncthreads();  // the stages' last reads
+    for (unsigned left = bad; left; left &= left - 1) {
+      const int su = __ffs(left) - 1;
+      const int px = X0 + (warp & 3) * 4 + (lane & 3);
+      const int py = Y0 + (warp >> 2) * 4 + ((lane >> 2) & 3);
+      float sum = 0.f;
+      if (px < g && py < g) {
+        int tile, tl;
+        pixel_tile(px, py, A.M.tiles_x, A.M.tw_shift, &tile, &tl);
+        sum = slow_sum<LK, FK == FK_HALF>(A, dl + ((int64_t)tile * 128 + tl * 4) * W, px, py,
+                                          lane >> 4, unit_base, su);
+      }
+      sum = fadd(sum, __shfl_xor_sync(0xffffffffu, sum, 16));
+      if (lane < 16) again[lane * U + su] = sum;
+    }
+    __syncwarp();
+  }
+
   // ---- epilogue: the lane holds columns 2 t and 2 t + 1 of every accumulator
   // tile for its two pixels; column n of tile j is slice 8 j + n of the unit
   // with halves (NV vectors of N = 2 slices), n * NT + j with TF32 (one vector
@@ -616,14 +661,12 @@ __device__ __forceinline__ void backward_mma_block(const IterArgs& A, int unit, 
     if constexpr (FK == FK_SPLIT) {
 #pragma unroll
       for (int j = 0; j < N; ++j)
-        if (j < n) num[j] *= 1.f / split_scale(A.F.fmax[s0 + j]);
+        if (j < n) num[j] *= 1.f / split_scale(A.F.stat[s0 + j].most);
     }
-    if (!finite) {
+    if (bad) {
 #pragma unroll
       for (int j = 0; j < N; ++j)
-        if (j < n)
-          num[j] = slow_sum<LK, FK == FK_HALF>(A, dl + ((int64_t)tile * 128 + tl * 4) * W, x, y,
-                                               unit_base, su + j);
+        if (bad >> (su + j) & 1u) num[j] = again[(row + 8 * h) * U + su + j];
     }
     if constexpr (LK == LK_U16) {
 #pragma unroll

@@ -151,22 +151,24 @@ enum BackEpi { EPI_UPDATE = 0, EPI_REPLICA = 1 };
 // reads them: units of U = 8, 16 or 32 slices, each [P4][RP][U] floats or
 // halves with kRayPad zero columns before column 0 of an angle and twice as
 // many after the last (windows may start and end outside the detector).
-// flags[b] != 0: slice batch b holds a non-finite factor on a ray with
-// segments (reset by the batch's forward launch, raised by its finish).
+// Per slice, reset by the slice's forward launch and raised by its finish: bad
+// != 0 where a factor of a ray with segments is not finite; the bits of the
+// largest |factor| (split plans).
 constexpr int kRayPad = 8;
+struct FactorStat {
+  unsigned most;
+  int bad;
+};
 // Float factors of plans with f16 lengths are also kept as two halves each,
 // [P4][RP][2][U] (high parts, then low), scaled per slice by
-// split_scale(fmax[slice]); fmax: bits of the slice's largest |factor|,
-// reset and raised as the flags are.
+// split_scale(stat[slice].most).
 struct FactorDev {
   void* base;
   __half* split;
-  unsigned* fmax;
   int64_t unit_elems;  // P4 * RP * U
   int U, RP;
   int ring;            // units held; unit u is at u % ring
-  int* flags;
-  int nflags;          // slice batches
+  FactorStat* stat;    // [slices, rounded up to whole batches]
   int blocks_x;        // 16 x 8 pixel blocks per row
 };
 // at least the 21 columns that a block stages
@@ -232,8 +234,7 @@ struct FwdItem {
   TileMatrixDev T;
   const float* recon;   // the batch's reconstruction slots
   float* part;          // the plan's partial-sum slots
-  int* flag;            // the batch's non-finite flag (nullptr: none), reset here
-  unsigned* fmax;       // and its slices' largest factors (nullptr: none)
+  FactorStat* stat;     // of the batch's slices (nullptr: none), reset here
   int g;
   float inv_scale;
   int64_t first;
@@ -466,11 +467,10 @@ void launch_runs_fill(const DevGeom& G, const MatrixDev& M, int tiles_x, int ts,
                       const int64_t* gseg_off, const int64_t* gcode_off,
                       void* tlen, uint32_t* tcode, cudaStream_t st);
 // part: [runs][K] partial sums, written (not accumulated) by each launch;
-// flag, fmax (optional): the batch's non-finite flag and its K slices'
-// largest factors, reset; width: A.K slices, or the 8 of 8 / A.K batches (half
-// tile, not compensated)
+// stat (optional): of the batch's slices, reset; width: A.K slices, or the 8 of
+// 8 / A.K batches (half tile, not compensated)
 void launch_forward_tiled(const IterArgs& A, const TileMatrixDev& T,
-                          const float* recon_batch, float* part, int* flag, unsigned* fmax,
+                          const float* recon_batch, float* part, FactorStat* stat,
                           int width, cudaStream_t st);
 // ray sums from the partial sums (fixed order) -> per-ray values `out`
 void launch_fwd_finish(const IterArgs& A, const TileMatrixDev& T, const float* part,
@@ -508,8 +508,8 @@ void launch_strips_fill(const DevGeom& G, const MatrixDev& M, const StripDev& S,
                         uint32_t* meta, uint8_t* grazed, StripExc* exc, int exc_cap, int* nexc,
                         cudaStream_t st);
 // U (32 or 64) slices from slice `first`: their halves into img ([pixel][U]),
-// then every bundle's sums into part ([bundle][16][U]); reset: the flags and
-// largest factors of their batches too
+// then every bundle's sums into part ([bundle][16][U]); reset: their
+// factors' stat too
 void launch_strips_forward(const IterArgs& A, const StripDev& S, int first, int U,
                            const float* recon, __half* img, float* part, int reset,
                            cudaStream_t st);

@@ -66,7 +66,7 @@ struct tg_plan {
   bool mma = false;
   FactorDev F[2] = {};
   int unit = 0, nunits = 0, group_units = 1;  // slices per unit, units, units per group
-  int* d_flags = nullptr;
+  FactorStat* d_stat = nullptr;  // per slice
   cudaEvent_t ev_meet = nullptr, ev_group[2] = {nullptr, nullptr};
   // strip-ordered forward (in place of the tile-ordered one): a group's halves
   // of the reconstruction and bundle sums
@@ -870,16 +870,13 @@ int ensure_factors(tg_plan* p, bool half) {
   f.unit_elems = (int64_t)p->M.P4 * f.RP * f.U;
   f.ring = std::min(p->nunits, 2 * p->group_units);
   f.blocks_x = (p->C + 15) / 16;
-  f.nflags = p->nb;
-  if (!p->d_flags) TG_TRY(dalloc(p, &p->d_flags, (size_t)p->nb, true));
-  f.flags = p->d_flags;
+  if (!p->d_stat) TG_TRY(dalloc(p, &p->d_stat, (size_t)p->nb * p->K, true));
+  f.stat = p->d_stat;
   char* base = nullptr;
   TG_TRY(dalloc(p, &base, (size_t)f.unit_elems * f.ring * (half ? 2 : 4), true));
   f.base = base;
-  if (!half && p->M.dlen_kind == LK_F16) {
+  if (!half && p->M.dlen_kind == LK_F16)
     TG_TRY(dalloc(p, &f.split, (size_t)f.unit_elems * f.ring * 2, true));
-    TG_TRY(dalloc(p, &f.fmax, (size_t)p->nb * p->K, true));
-  }
   F = f;
   return TG_OK;
 }
@@ -1591,7 +1588,7 @@ static int run_forward(tg_plan* p, const IterArgs& A0, int b, int nb, int out_mo
     A.half_factors = 0;
     {
       Timed t(p, 0);
-      launch_forward_tiled(A, p->T, src, p->d_part, nullptr, nullptr, p->K, p->st);
+      launch_forward_tiled(A, p->T, src, p->d_part, nullptr, p->K, p->st);
     }
     Timed t(p, 2);
     launch_fwd_finish(A, p->T, p->d_part,
@@ -1671,7 +1668,7 @@ static void issue_units(tg_plan* p, IterArgs A, int mode, bool two, int epi,
       {
         Timed t(p, 0);
         launch_forward_tiled(A, p->T, batch_ptr(p, p->d_recon[p->cur], b * p->K + p->fshift),
-                             part, p->d_flags + b, A.F.split ? A.F.fmax + b * p->K : nullptr,
+                             part, A.F.stat + b * p->K,
                              nb * p->K, st[odd]);
       }
       Timed t(p, 2);
@@ -1730,7 +1727,7 @@ static void issue_iteration(tg_plan* p, const IterArgs& A0, int mode, bool two_s
       const float* src = batch_ptr(p, p->d_recon[p->cur], b * p->K + p->fshift);
       {
         Timed t(p, 0);
-        launch_forward_tiled(A, p->T, src, part, nullptr, nullptr, p->K, s);
+        launch_forward_tiled(A, p->T, src, part, nullptr, p->K, s);
       }
       Timed t(p, 2);
       launch_fwd_finish(A, p->T, part, p->d_sino + (int64_t)b * p->R * p->K, upd, mode, s);
@@ -2004,8 +2001,7 @@ void multi_build(const tg_batch* b, const int* algs, const tg_params* params, in
         f.T = p->T;
         f.recon = batch_ptr(p, p->d_recon[cur], r * p->K + p->fshift);
         f.part = p->d_part;
-        f.flag = p->mma ? p->d_flags + r : nullptr;
-        f.fmax = A.F.split ? A.F.fmax + r * p->K : nullptr;
+        f.stat = p->mma ? A.F.stat + r * p->K : nullptr;
         f.g = p->C;
         f.inv_scale = A.M.inv_scale;
         f.first = p->T.ntiles;  // block count; turned into offsets below

@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(kStripBlock, 1)
 
 // One warp per ray (grid-strided): its chunks' sums in order (lane = U / 32
 // slices), the exceptions, then the per-ray value of every slice: factors into
-// F's units (half or float, with the flags and largest factors of
+// F's units (half or float, with the stat of
 // finish_units_ray), or the ray sums (sim).
 template <int U, bool FH>
 __global__ void __launch_bounds__(kFinishWarps * 32)
@@ -649,10 +649,10 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
       if constexpr (FH) {
         const __half h = __float2half_rn(o);
         reinterpret_cast<__half*>(F.base)[e] = h;
-        if (!(fabsf(__half2float(h)) < 7e4f)) F.flags[s / K] = 1;
+        if (!(fabsf(__half2float(h)) < 7e4f)) F.stat[s].bad = 1;
       } else {
         reinterpret_cast<float*>(F.base)[e] = o;
-        if (!(fabsf(o) < 1e38f)) F.flags[s / K] = 1;
+        if (!(fabsf(o) < 1e38f)) F.stat[s].bad = 1;
         most[k] = fmaxf(most[k], fabsf(o));
       }
     }
@@ -668,20 +668,16 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
         float m = 0.f;
         for (int w = 0; w < kFinishWarps; ++w) m = fmaxf(m, s_most[w][k]);
         const int s = first + k;
-        if (s < nslices && m > 0.f) atomicMax(F.fmax + s, __float_as_uint(m));
+        if (s < nslices && m > 0.f) atomicMax(&F.stat[s].most, __float_as_uint(m));
       }
     }
   }
 }
 
-// Resets `bad`, and the flags and largest factors of batches b0 .. b1 - 1.
-__global__ void k_strips_reset(int* bad, int* flags, unsigned* fmax, int b0, int b1, int K) {
+// Resets `bad` and the stat of n slices.
+__global__ void k_strips_reset(int* bad, FactorStat* stat, int n) {
   if (threadIdx.x == 0) *bad = 0;
-  for (int i = b0 + threadIdx.x; i < b1; i += blockDim.x) {
-    flags[i] = 0;
-    if (fmax)
-      for (int k = 0; k < K; ++k) fmax[i * K + k] = 0u;
-  }
+  for (int i = threadIdx.x; i < n; i += blockDim.x) stat[i] = FactorStat{};
 }
 
 template <int NT>
@@ -719,9 +715,7 @@ void launch_strips_forward(const IterArgs& A, const StripDev& S, int first, int 
                            cudaStream_t st) {
   const int g = A.G.C;
   const int64_t g2 = (int64_t)g * g;
-  const int b0 = first / A.K;
-  const int b1 = reset ? min((A.S + A.K - 1) / A.K, (first + U) / A.K) : b0;
-  k_strips_reset<<<1, 256, 0, st>>>(S.bad, A.F.flags, A.F.split ? A.F.fmax : nullptr, b0, b1, A.K);
+  k_strips_reset<<<1, 64, 0, st>>>(S.bad, A.F.stat + first, reset ? min(U, A.S - first) : 0);
   const int64_t n = g2 * (U / 8);
   k_strips_image<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(recon, img, g2, A.K, U, A.S,
                                                              A.fshift, first, n, A.M.W, S.grazed, S.bad);

@@ -425,13 +425,10 @@ template <int K, int LK, bool H, bool COMP>
 __device__ __forceinline__ void forward_tiled_block(const TileMatrixDev& T, int g,
                                                     float inv_scale, int splits, int block,
                                                     const float* __restrict__ recon,
-                                                    float* __restrict__ part, int* flag,
-                                                    unsigned* fmax, int sk) {
+                                                    float* __restrict__ part,
+                                                    FactorStat* stat, int sk) {
   extern __shared__ float4 smem4[];
-  if (block == 0 && threadIdx.x < K) {
-    if (flag && threadIdx.x < K / sk) flag[threadIdx.x] = 0;
-    if (fmax) fmax[threadIdx.x] = 0u;
-  }
+  if (stat && block == 0 && threadIdx.x < K) stat[threadIdx.x] = FactorStat{};
   float* sm = reinterpret_cast<float*>(smem4);
   __half* smh = reinterpret_cast<__half*>(smem4);
   // `splits` blocks share a tile (small grids: fewer tiles than SMs); each
@@ -507,10 +504,9 @@ __device__ __forceinline__ void forward_tiled_block(const TileMatrixDev& T, int 
 template <int K, int LK, bool H, bool COMP>
 __global__ void __launch_bounds__(kBlock)
     k_forward_tiled(TileMatrixDev T, int g, float inv_scale, int splits,
-                    const float* __restrict__ recon, float* __restrict__ part, int* flag,
-                    unsigned* fmax, int sk) {
-  forward_tiled_block<K, LK, H, COMP>(T, g, inv_scale, splits, blockIdx.x, recon, part, flag,
-                                      fmax, sk);
+                    const float* __restrict__ recon, float* __restrict__ part, FactorStat* stat,
+                    int sk) {
+  forward_tiled_block<K, LK, H, COMP>(T, g, inv_scale, splits, blockIdx.x, recon, part, stat, sk);
 }
 
 // Many plans' forward projections in one launch: block -> work item (a
@@ -520,7 +516,7 @@ __global__ void __launch_bounds__(kBlock)
     k_forward_tiled_multi(const FwdItem* __restrict__ items, int nitems) {
   const FwdItem& it = items[item_of(items, nitems, blockIdx.x)];
   forward_tiled_block<K, LK, H, COMP>(it.T, it.g, it.inv_scale, 1,
-                                      (int)(blockIdx.x - it.first), it.recon, it.part, it.flag, it.fmax, K);
+                                      (int)(blockIdx.x - it.first), it.recon, it.part, it.stat, K);
 }
 
 // A ray's sums: its partial sums (its runs' slots) added in path order.
@@ -586,7 +582,7 @@ __device__ __forceinline__ void fwd_finish_ray(int64_t r, const int* __restrict_
 
 // The same into the units of the tensor-core backprojection (FactorDev).
 // Rays without segments store 0 (no pixel uses them); a non-finite factor
-// raises its batch's flag. sk: slices per pass, 8 / sk batches at K = 8 (R rays
+// marks its slice. sk: slices per pass, 8 / sk batches at K = 8 (R rays
 // between their rows of the sinogram).
 template <int K, bool FH>
 __device__ __forceinline__ void finish_units_ray(int64_t r, int64_t R, int sk,
@@ -635,13 +631,13 @@ __device__ __forceinline__ void finish_units_ray(int64_t r, int64_t R, int sk,
       for (int j = 0; j < K; ++j) {
         const unsigned act = __activemask();
         const unsigned m = __reduce_max_sync(act, __float_as_uint(fabsf(o.v[j])));
-        if ((threadIdx.x & 31) == __ffs(act) - 1 && m > F.fmax[batch * sk + j])
-          atomicMax(F.fmax + batch * sk + j, m);
+        unsigned* most = &F.stat[batch * sk + j].most;
+        if ((threadIdx.x & 31) == __ffs(act) - 1 && m > *most) atomicMax(most, m);
       }
     }
   }
-  for (int b = 0; bad; ++b, bad >>= sk)
-    if (bad & ((1u << sk) - 1u)) F.flags[batch + b] = 1;
+  for (int s = batch * sk; bad; ++s, bad >>= 1)
+    if (bad & 1u) F.stat[s].bad = 1;
 }
 
 // Float factors of one column and 8 slices -> high and low halves (FactorDev).
@@ -659,7 +655,7 @@ __device__ __forceinline__ void split_factors(const FactorDev& F, int P4, int S,
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int s = unit * F.U + o * 8 + j;
-    const float x = v.v[j] * (s < S ? split_scale(F.fmax[s]) : 1.f);
+    const float x = v.v[j] * (s < S ? split_scale(F.stat[s].most) : 1.f);
     hi.v[j] = __half2float(__float2half_rn(x));
     lo.v[j] = fsub(x, hi.v[j]);
   }
@@ -729,7 +725,7 @@ __global__ void k_fwd_finish_multi(const FinItem* __restrict__ items, int nitems
 
 template <int K, int LK, bool H, bool COMP>
 void fwd_tiled_launch(const TileMatrixDev& T, int g, float inv_scale,
-                      const float* recon, float* part, int* flag, unsigned* fmax, int sk,
+                      const float* recon, float* part, FactorStat* stat, int sk,
                       cudaStream_t st) {
   const int smem = TilePlanes<K, H>::bytes(T.ts);
   cudaFuncSetAttribute(k_forward_tiled<K, LK, H, COMP>,
@@ -740,15 +736,15 @@ void fwd_tiled_launch(const TileMatrixDev& T, int g, float inv_scale,
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int splits = max(1, min(16, (2 * sms + T.ntiles - 1) / T.ntiles));
   k_forward_tiled<K, LK, H, COMP><<<T.ntiles * splits, T.bw * 32, smem, st>>>(
-      T, g, inv_scale, splits, recon, part, flag, fmax, sk);
+      T, g, inv_scale, splits, recon, part, stat, sk);
 }
 
 template <int K, bool H, bool COMP>
 void fwd_tiled_kind(const TileMatrixDev& T, int g, int len_kind, float inv_scale,
-                    const float* recon, float* part, int* flag, unsigned* fmax, int sk,
+                    const float* recon, float* part, FactorStat* stat, int sk,
                     cudaStream_t st) {
 #define TG_TILED(LKK) \
-  fwd_tiled_launch<K, LKK, H, COMP>(T, g, inv_scale, recon, part, flag, fmax, sk, st)
+  fwd_tiled_launch<K, LKK, H, COMP>(T, g, inv_scale, recon, part, stat, sk, st)
   switch (len_kind) {
     case LK_F32: TG_TILED(LK_F32); break;
     case LK_BF16: TG_TILED(LK_BF16); break;
@@ -760,24 +756,24 @@ void fwd_tiled_kind(const TileMatrixDev& T, int g, int len_kind, float inv_scale
 
 template <int K, bool COMP>
 void fwd_tiled_half(const IterArgs& A, const TileMatrixDev& T, const float* recon,
-                    float* part, int* flag, unsigned* fmax, cudaStream_t st) {
+                    float* part, FactorStat* stat, cudaStream_t st) {
   // an f32 tile of 16 slices would not fit shared memory (plan creation
   // requires half_gathers with 16 slices per pass and forward_tiles)
   if (K == 16 || A.half_tile)
-    fwd_tiled_kind<K, true, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, flag, fmax,
+    fwd_tiled_kind<K, true, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, stat,
                                   A.K, st);
   else if constexpr (K != 16)
-    fwd_tiled_kind<K, false, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, flag, fmax,
+    fwd_tiled_kind<K, false, COMP>(T, A.G.C, A.M.len_kind, A.M.inv_scale, recon, part, stat,
                                    A.K, st);
 }
 
 // compensated sums: up to 8 slices per pass (plan creation checks)
 template <int K>
 void fwd_tiled_comp(const IterArgs& A, const TileMatrixDev& T, const float* recon,
-                    float* part, int* flag, unsigned* fmax, cudaStream_t st) {
+                    float* part, FactorStat* stat, cudaStream_t st) {
   constexpr bool kComp = K <= 8;
-  if (kComp && A.comp) fwd_tiled_half<K, kComp>(A, T, recon, part, flag, fmax, st);
-  else fwd_tiled_half<K, false>(A, T, recon, part, flag, fmax, st);
+  if (kComp && A.comp) fwd_tiled_half<K, kComp>(A, T, recon, part, stat, st);
+  else fwd_tiled_half<K, false>(A, T, recon, part, stat, st);
 }
 
 inline int blocks_for(int64_t n, int b) { return (int)((n + b - 1) / b); }
@@ -905,14 +901,14 @@ void launch_runs_fill(const DevGeom& G, const MatrixDev& M, int tiles_x, int ts,
 }
 
 void launch_forward_tiled(const IterArgs& A, const TileMatrixDev& T,
-                          const float* recon_batch, float* part, int* flag, unsigned* fmax,
+                          const float* recon_batch, float* part, FactorStat* stat,
                           int width, cudaStream_t st) {
   switch (width) {
-    case 1: fwd_tiled_comp<1>(A, T, recon_batch, part, flag, fmax, st); break;
-    case 2: fwd_tiled_comp<2>(A, T, recon_batch, part, flag, fmax, st); break;
-    case 4: fwd_tiled_comp<4>(A, T, recon_batch, part, flag, fmax, st); break;
-    case 8: fwd_tiled_comp<8>(A, T, recon_batch, part, flag, fmax, st); break;
-    default: fwd_tiled_comp<16>(A, T, recon_batch, part, flag, fmax, st); break;
+    case 1: fwd_tiled_comp<1>(A, T, recon_batch, part, stat, st); break;
+    case 2: fwd_tiled_comp<2>(A, T, recon_batch, part, stat, st); break;
+    case 4: fwd_tiled_comp<4>(A, T, recon_batch, part, stat, st); break;
+    case 8: fwd_tiled_comp<8>(A, T, recon_batch, part, stat, st); break;
+    default: fwd_tiled_comp<16>(A, T, recon_batch, part, stat, st); break;
   }
 }
 
