@@ -139,7 +139,8 @@ struct StripDev {
   const int* exc_first;    // [P*C + 1] exceptions per ray, or nullptr
   const StripExc* exc;
   const uint8_t* grazed;   // [C*C] 1: a ray's zero-length segment lies in the pixel
-  int* bad;                // a crossed pixel's half is not finite
+  int* bad;                // [64] slices of the launch: a crossed pixel's half is not
+                           // finite; [1] blocks that are done with these marks
 };
 
 // Which per-ray value the forward kernel stores.

@@ -764,7 +764,7 @@ int build_strips(tg_plan* p, const StripTables& T) {
   constexpr int kCap = 1 << 20;
   if (!keep(&cls, P, false) || !keep(&place, P, false) || !keep(&cls16, S.nblk16, false) ||
       !keep(&al, alpha.size(), false) || !keep(&sg, P, false) || !keep(&b16, S.nblk16, false) ||
-      !keep(&quad, T.quad.size(), false) || !keep(&S.bad, 1, true) ||
+      !keep(&quad, T.quad.size(), false) || !keep(&S.bad, 65, true) ||
       !keep(&grazed, p->g2, true) || !keep(&codes, nsteps * 64, true) ||
       !keep(&meta, nsteps * 16, false) ||
       !keep(&p->d_simg, U * p->g2, false) || !keep(&p->d_spart, U * S.nbundles * 16, false))

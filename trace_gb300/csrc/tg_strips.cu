@@ -320,13 +320,15 @@ __global__ void __launch_bounds__(128)
 // FP32 reconstruction slots -> halves [pixel][U]; one thread per pixel
 // and 8 slices. A product runs over whole windows, so a non-finite pixel would
 // reach rays beside it: one that no ray crosses, not even with a zero length
-// (0 / 0 in the updates), becomes 0; any other raises `bad`, and the finish
-// kernel then walks the rays.
+// (0 / 0 in the updates), becomes 0; any other marks its slice in `bad`, and the
+// rays of that slice are then walked. Resets the stat of nstat slices.
 __global__ void k_strips_image(const float* __restrict__ recon, __half* __restrict__ img,
                                int64_t g2, int K, int U, int S, int first_slot, int first,
                                int64_t n, const float* __restrict__ W,
-                               const uint8_t* __restrict__ grazed, int* bad) {
+                               const uint8_t* __restrict__ grazed, int* bad,
+                               FactorStat* stat, int nstat) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.x == 0 && threadIdx.x < nstat) stat[threadIdx.x] = FactorStat{};
   if (i >= n) return;
   const int oct = U / 8;
   const int o = (int)(i % oct);
@@ -351,10 +353,12 @@ __global__ void k_strips_image(const float* __restrict__ recon, __half* __restri
   }
   if (!finite) {
     const bool crossed = W[p] != 0.f || grazed[p];
-    if (crossed) *bad = 1;
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (!crossed && !(fabsf(v.v[j]) < 7e4f)) v.v[j] = 0.f;
+    for (int j = 0; j < 8; ++j) {
+      if (fabsf(v.v[j]) < 7e4f) continue;
+      if (crossed) bad[o * 8 + j] = 1;
+      else v.v[j] = 0.f;
+    }
   }
   store_hvec<8>(img + p * U + o * 8, v);
 }
@@ -556,26 +560,91 @@ __global__ void __launch_bounds__(kStripBlock, 1)
   }
 }
 
+// Stores the per-ray value of slice s from its sum v (b: the sinogram's value, at:
+// its place there); returns |factor|.
+template <bool FH>
+__device__ __forceinline__ float ray_value(const FactorDev& F, float* sim, int64_t at, int a,
+                                           int c, int n, int s, float v, float b, float a2,
+                                           int out_mode, float fofs) {
+  if (out_mode == FWD_SIM) {
+    sim[at] = v;
+    return 0.f;
+  }
+  float o = 0.f;
+  if (n > 0) {
+    o = out_mode == FWD_SIRT ? fdiv(fsub(b, v), a2) : fdiv(b, v);
+    if constexpr (FH) o -= fofs;
+  }
+  const int u = s / F.U;
+  const int64_t e = factor_at((int64_t)(u % F.ring) * F.unit_elems, F.RP, F.U, a, c, s % F.U);
+  if constexpr (FH) {
+    const __half h = __float2half_rn(o);
+    reinterpret_cast<__half*>(F.base)[e] = h;
+    if (!(fabsf(__half2float(h)) < 7e4f)) F.stat[s].bad = 1;
+  } else {
+    reinterpret_cast<float*>(F.base)[e] = o;
+    if (!(fabsf(o) < 1e38f)) F.stat[s].bad = 1;
+  }
+  return fabsf(o);
+}
+
+// The marked slices' rays, walked: one of a warp's 32 rays per lane. The last
+// block clears the marks for the next launch.
+template <bool FH>
+__global__ void __launch_bounds__(kFinishWarps * 32)
+    k_strips_walk(const __grid_constant__ DevGeom G, const __grid_constant__ MatrixDev M,
+                  const __grid_constant__ FactorDev F, int src, int* bad,
+                  const __half* __restrict__ img, const float* __restrict__ sino,
+                  float* __restrict__ sim, int U, int first, int nslices, int64_t K, int out_mode,
+                  float fofs) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nrays = (int64_t)G.P * G.C;
+  for (int k = 0; k < U; k += 32)
+    for (unsigned left = __ballot_sync(0xffffffffu, bad[k + lane] != 0); left; left &= left - 1) {
+      const int su = k + __ffs(left) - 1, s = first + su;
+      if (s >= nslices) continue;
+      float most = 0.f;
+      for (int64_t grp = (int64_t)blockIdx.x * kFinishWarps + (threadIdx.x >> 5);
+           grp < (int64_t)G.P * G.gpa; grp += (int64_t)gridDim.x * kFinishWarps) {
+        const int a = (int)(grp / G.gpa), c = (int)(grp - (int64_t)a * G.gpa) * 32 + lane;
+        if (c >= G.C) continue;
+        const int64_t r = (int64_t)a * G.C + c, at = s / K * nrays * K + r * K + s % K;
+        most = fmaxf(most, ray_value<FH>(F, sim, at, a, c, M.rnseg[r], s,
+                                         walk_ray(G, M, src, r, img + su, U),
+                                         out_mode != FWD_SIM ? __ldg(sino + at) : 0.f,
+                                         out_mode == FWD_SIRT ? M.ra2[r] : 1.f, out_mode, fofs));
+      }
+      if (!FH && out_mode != FWD_SIM && F.split && most > 0.f)
+        atomicMax(&F.stat[s].most, __float_as_uint(most));
+    }
+  __syncthreads();  // the block has read the marks
+  if (threadIdx.x == 0 && atomicAdd(bad + 64, 1) == (int)gridDim.x - 1)
+    for (int i = 0; i <= 64; ++i) bad[i] = 0;
+}
+
 // One warp per ray (grid-strided): its chunks' sums in order (lane = U / 32
 // slices), the exceptions, then the per-ray value of every slice: factors into
-// F's units (half or float, with the stat of
-// finish_units_ray), or the ray sums (sim).
+// F's units (half or float, with the stat of finish_units_ray), or the ray sums
+// (sim). Slices marked in `bad` are k_strips_walk's.
 template <int U, bool FH>
 __global__ void __launch_bounds__(kFinishWarps * 32)
     k_strips_finish(const __grid_constant__ DevGeom G, const __grid_constant__ MatrixDev M,
                     const __grid_constant__ StripDev S, const __grid_constant__ FactorDev F,
-                    int src, const int* __restrict__ bad, const float* __restrict__ part,
+                    const int* __restrict__ bad, const float* __restrict__ part,
                     const __half* __restrict__ img, const float* __restrict__ sino,
                     float* __restrict__ sim, int first, int nslices, int K, int out_mode,
                     float fofs) {
   constexpr int N = U / 32;
-  const bool walk = *bad != 0;
   const int lane = threadIdx.x & 31;
   const int64_t nrays = (int64_t)G.P * G.C;
   const int s0 = first + lane * N;  // the lane's slices
   float most[N];
+  unsigned walk = 0;  // a bit per slice of the lane
 #pragma unroll
-  for (int k = 0; k < N; ++k) most[k] = 0.f;
+  for (int k = 0; k < N; ++k) {
+    most[k] = 0.f;
+    walk |= bad[lane * N + k] ? 1u << k : 0u;
+  }
   const int64_t w0 = (int64_t)blockIdx.x * kFinishWarps + (threadIdx.x >> 5);
   for (int64_t r = w0; r < nrays; r += (int64_t)gridDim.x * kFinishWarps) {
     const int a = (int)(r / G.C), c = (int)(r - (int64_t)a * G.C);
@@ -591,11 +660,7 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
                  ? __ldg(sino + (int64_t)(s / K) * nrays * K + r * K + s % K)
                  : 0.f;
     }
-    if (walk) {
-#pragma unroll
-      for (int k = 0; k < N; ++k) v[k] = walk_ray(G, M, src, r, img + lane * N + k, U);
-    }
-    for (int j0 = 0; n > 0 && !walk && j0 < S.nchunks; j0 += 32) {
+    for (int j0 = 0; n > 0 && j0 < S.nchunks; j0 += 32) {
       // the ray's row of sums in chunk j0 + lane
       int64_t at = -1;
       if (j0 + lane < S.nchunks) {
@@ -620,7 +685,7 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
           for (int k = 0; k < N; ++k) v[k] = fadd(v[k], q[i].v[k]);
       }
     }
-    if (S.exc_first && !walk) {
+    if (S.exc_first) {
       for (int e = S.exc_first[r]; e < S.exc_first[r + 1]; ++e) {
         const StripExc x = S.exc[e];
         const float l = (float)x.code * M.inv_scale;
@@ -633,28 +698,10 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
 #pragma unroll
     for (int k = 0; k < N; ++k) {
       const int s = s0 + k;
-      if (s >= nslices) continue;
+      if (s >= nslices || (walk >> k & 1u)) continue;
       const int64_t at = (int64_t)(s / K) * nrays * K + r * K + s % K;
-      if (out_mode == FWD_SIM) {
-        sim[at] = v[k];
-        continue;
-      }
-      float o = 0.f;
-      if (n > 0) {
-        o = out_mode == FWD_SIRT ? fdiv(fsub(b[k], v[k]), a2) : fdiv(b[k], v[k]);
-        if constexpr (FH) o -= fofs;
-      }
-      const int u = s / F.U;
-      const int64_t e = factor_at((int64_t)(u % F.ring) * F.unit_elems, F.RP, F.U, a, c, s % F.U);
-      if constexpr (FH) {
-        const __half h = __float2half_rn(o);
-        reinterpret_cast<__half*>(F.base)[e] = h;
-        if (!(fabsf(__half2float(h)) < 7e4f)) F.stat[s].bad = 1;
-      } else {
-        reinterpret_cast<float*>(F.base)[e] = o;
-        if (!(fabsf(o) < 1e38f)) F.stat[s].bad = 1;
-        most[k] = fmaxf(most[k], fabsf(o));
-      }
+      const float f = ray_value<FH>(F, sim, at, a, c, n, s, v[k], b[k], a2, out_mode, fofs);
+      if constexpr (!FH) most[k] = fmaxf(most[k], f);
     }
   }
   if constexpr (!FH) {
@@ -672,12 +719,6 @@ __global__ void __launch_bounds__(kFinishWarps * 32)
       }
     }
   }
-}
-
-// Resets `bad` and the stat of n slices.
-__global__ void k_strips_reset(int* bad, FactorStat* stat, int n) {
-  if (threadIdx.x == 0) *bad = 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) stat[i] = FactorStat{};
 }
 
 template <int NT>
@@ -715,10 +756,11 @@ void launch_strips_forward(const IterArgs& A, const StripDev& S, int first, int 
                            cudaStream_t st) {
   const int g = A.G.C;
   const int64_t g2 = (int64_t)g * g;
-  k_strips_reset<<<1, 64, 0, st>>>(S.bad, A.F.stat + first, reset ? min(U, A.S - first) : 0);
   const int64_t n = g2 * (U / 8);
   k_strips_image<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(recon, img, g2, A.K, U, A.S,
-                                                             A.fshift, first, n, A.M.W, S.grazed, S.bad);
+                                                             A.fshift, first, n, A.M.W, S.grazed, S.bad,
+                                                             A.F.stat + first,
+                                                             reset ? min(U, A.S - first) : 0);
   const float scale = A.M.inv_scale * 256.f;
   if (U == 64)
     forward_strips<8>(S, g, scale, img, part, st);
@@ -734,8 +776,8 @@ void launch_strips_finish(const IterArgs& A, const StripDev& S, int first, int U
   const unsigned bx = (unsigned)std::min<int64_t>((rays + kFinishWarps - 1) / kFinishWarps, 152 * 32);
 #define TG_FIN(UU, FH)                                                                       \
   k_strips_finish<UU, FH><<<bx, kFinishWarps * 32, 0, st>>>(                                 \
-      A.G, A.M, S, A.F, seg_source(A.M), S.bad, part, img, sino, sim, first, A.S, A.K,       \
-      out_mode, factor_offset(A.half_factors))
+      A.G, A.M, S, A.F, S.bad, part, img, sino, sim, first, A.S, A.K, out_mode,              \
+      factor_offset(A.half_factors))
   const bool fh = A.half_factors != FACT_F32 && out_mode == FWD_RATIO;
   if (U == 64) {
     if (fh) TG_FIN(64, true); else TG_FIN(64, false);
@@ -743,6 +785,12 @@ void launch_strips_finish(const IterArgs& A, const StripDev& S, int first, int U
     if (fh) TG_FIN(32, true); else TG_FIN(32, false);
   }
 #undef TG_FIN
+#define TG_WALK(FH)                                                                        \
+  k_strips_walk<FH><<<(unsigned)std::min<int64_t>(bx, 152 * 4), kFinishWarps * 32, 0, st>>>( \
+      A.G, A.M, A.F, seg_source(A.M), S.bad, img, sino, sim, U, first, A.S, A.K, out_mode,   \
+      factor_offset(A.half_factors))
+  if (fh) TG_WALK(true); else TG_WALK(false);
+#undef TG_WALK
 }
 
 }  // namespace tg
