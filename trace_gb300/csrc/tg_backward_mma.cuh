@@ -52,7 +52,9 @@
 // not cross: the finish kernel marks the slice when it stores a non-finite
 // factor for a ray with segments, and the kernel then takes that slice's sums
 // per crossed ray (slow_sum), as the scalar kernel does. The columns of a
-// product are independent, so the other slices' stay.
+// product are independent, so the other slices' stay. The same goes for
+// FK_SPLIT's wide slices: where one hot ray's factor stands 2^15 and more over
+// most others, two halves of one scale keep less of these than FP32 does.
 //
 // Measured (1024 x 1024, 720 angles, ms per 8 slices; the scalar kernel of
 // tg_backward.cuh before the arrow): MLEM half factors 1.15 -> 0.96 in units
@@ -195,9 +197,9 @@ __device__ __forceinline__ void pair_lengths(const PairWord<LK>& w, float& l0, f
 }
 
 // Sum over the pixel's crossed rays of one slice, one product at a time, of
-// every other angle quad from q0 on (the path taken when a factor is not
-// finite): `at` is the pixel's first pair. The four angles' factors are in
-// flight together.
+// every other angle quad from q0 on: for slices that a matrix product does not
+// serve. `at` is the pixel's first pair. The four angles' factors are in flight
+// together.
 template <int LK, bool HALF>
 __device__ __noinline__ float slow_sum(const IterArgs& A, const uint32_t* at, int x, int y, int q0,
                                        int64_t unit_base, int su) {
@@ -240,10 +242,19 @@ __device__ __noinline__ float slow_sum(const IterArgs& A, const uint32_t* at, in
   return acc;
 }
 
-// A bit per slice of the unit: those with a non-finite factor.
-__device__ __forceinline__ unsigned bad_slices(const IterArgs& A, int unit, int lane) {
+// A bit per slice of the unit: those that the products do not serve. bad: a
+// non-finite factor. Wide (split plans): most factors lie below 2^-15 of the largest
+// one, with which they share a scale (or none is in the sample).
+template <bool SPLIT>
+__device__ __forceinline__ unsigned redo_slices(const IterArgs& A, int unit, int lane) {
   const int s = unit * A.F.U + lane;
-  return __ballot_sync(0xffffffffu, lane < A.F.U && s < A.S && A.F.stat[s].bad != 0);
+  bool redo = false;
+  if (lane < A.F.U && s < A.S) {
+    const FactorStat t = A.F.stat[s];
+    redo = t.bad != 0 ||
+           (SPLIT && (t.small > t.nonzero / 2 || (t.nonzero == 0u && t.most != 0u)));
+  }
+  return __ballot_sync(0xffffffffu, redo);
 }
 
 // n <= N consecutive slots' values of one pixel, slot s's at `r` (one vector
@@ -596,15 +607,15 @@ __device__ __forceinline__ void backward_mma_block(const IterArgs& A, int unit, 
     }
   }
 
-  // Slices with a non-finite factor: their sums again, ray by ray, into shared
+  // Slices that the products do not serve: their sums again, ray by ray, into shared
   // memory ([warp][16 pixels][U]; kept out of the accumulators' registers). A lane
   // takes one of the tile's 16 pixels and half of the angle quads.
-  const unsigned bad = bad_slices(A, unit, lane);
+  const unsigned redo = redo_slices<FK == FK_SPLIT>(A, unit, lane);
   float* const again = reinterpret_cast<float*>(sm) + warp * 16 * U;
   static_assert(kMmaTiles * 16 * U * 4 <= St::kBytes, "the sums fit the stages");
-  if (bad) {
+  if (redo) {
     __syncthreads();  // the stages' last reads
-    for (unsigned left = bad; left; left &= left - 1) {
+    for (unsigned left = redo; left; left &= left - 1) {
       const int su = __ffs(left) - 1;
       const int px = X0 + (warp & 3) * 4 + (lane & 3);
       const int py = Y0 + (warp >> 2) * 4 + ((lane >> 2) & 3);
@@ -663,10 +674,10 @@ __device__ __forceinline__ void backward_mma_block(const IterArgs& A, int unit, 
       for (int j = 0; j < N; ++j)
         if (j < n) num[j] *= 1.f / split_scale(A.F.stat[s0 + j].most);
     }
-    if (bad) {
+    if (redo) {
 #pragma unroll
       for (int j = 0; j < N; ++j)
-        if (bad >> (su + j) & 1u) num[j] = again[(row + 8 * h) * U + su + j];
+        if (redo >> (su + j) & 1u) num[j] = again[(row + 8 * h) * U + su + j];
     }
     if constexpr (LK == LK_U16) {
 #pragma unroll

@@ -153,16 +153,21 @@ enum BackEpi { EPI_UPDATE = 0, EPI_REPLICA = 1 };
 // halves with kRayPad zero columns before column 0 of an angle and twice as
 // many after the last (windows may start and end outside the detector).
 // Per slice, reset by the slice's forward launch and raised by its finish: bad
-// != 0 where a factor of a ray with segments is not finite; the bits of the
-// largest |factor| (split plans).
+// != 0 where a factor of a ray with segments is not finite; on split plans the
+// bits of the largest |factor|, and (counted by the split, in a sample) the
+// factors that are not zero and those of them below about 2^-15 of the largest.
 constexpr int kRayPad = 8;
-struct FactorStat {
+struct __align__(16) FactorStat {
   unsigned most;
   int bad;
+  unsigned nonzero, small;
 };
 // Float factors of plans with f16 lengths are also kept as two halves each,
 // [P4][RP][2][U] (high parts, then low), scaled per slice by
-// split_scale(stat[slice].most).
+// split_scale(stat[slice].most): every factor from 2^-15 of the largest on keeps
+// FP32's 24 bits, smaller ones what is above 2^-39 of the largest. A slice most
+// of whose factors are smaller (one hot ray) is summed ray by ray instead
+// (redo_slices).
 struct FactorDev {
   void* base;
   __half* split;
@@ -263,7 +268,7 @@ struct FinItem {
   FactorDev F;
   int batch, C;
   int P4, S;            // launch_split_factors_multi
-  int64_t nrays;
+  int64_t nrays;        // there: blocks per unit
   int64_t first;        // 256 rays a block
   int out_mode;
   int fh;               // factor storage (FACT_*)
@@ -483,8 +488,8 @@ void launch_fwd_finish_units(const IterArgs& A, const TileMatrixDev& T, const fl
 // units first .. first + nunits - 1 of A.F: floats -> scaled halves (A.F.split)
 void launch_split_factors(const IterArgs& A, int first, int nunits, cudaStream_t st);
 void launch_split_factors_multi(const FinItem* items, int n, int64_t blocks, cudaStream_t st);
-// blocks of a plan's item in the multi launch
-int64_t split_blocks(const FactorDev& F, int P4, int nunits);
+// blocks per unit of a plan's item in the multi launch
+int64_t split_blocks(const FactorDev& F, int P4);
 // the same over many plans' slice batches in one launch each (device item
 // arrays; blocks = the launch's total blocks; all items of one launch share
 // K, the tile side and precision and the summation; 16-bit fixed-point

@@ -2025,8 +2025,8 @@ void multi_build(const tg_batch* b, const int* algs, const tg_params* params, in
         if (A.F.split) {
           n.P4 = A.M.P4;
           n.S = p->S;
-          n.nrays = (int64_t)p->nunits * A.M.P4 * A.F.RP * (A.F.U / 8);
-          n.first = split_blocks(A.F, A.M.P4, p->nunits);
+          n.nrays = split_blocks(A.F, A.M.P4);
+          n.first = n.nrays * p->nunits;
           splits.push_back(n);
         }
         BackItem k{};

@@ -640,40 +640,74 @@ __device__ __forceinline__ void finish_units_ray(int64_t r, int64_t R, int sk,
     if (bad & 1u) F.stat[s].bad = 1;
 }
 
-// Float factors of one column and 8 slices -> high and low halves (FactorDev).
-// `i` counts (unit from `first`, angle, column, 8 slices).
-__device__ __forceinline__ void split_factors(const FactorDev& F, int P4, int S, int first,
-                                              int64_t i) {
+// Float factors of one unit -> high and low halves (FactorDev); a thread takes 8
+// slices of one column, in block `block` of the unit's nblocks. Some 48 blocks
+// that a hash picks count FactorStat's nonzero and small (by all blocks, their
+// atomics would take longer than the rest: 400 columns, 300 angles, 24 slices 15.8
+// us, 7.7 without counting).
+constexpr int kSplitBlock = 256;
+
+__device__ __forceinline__ void split_unit(const FactorDev& F, int P4, int S, int unit, int block,
+                                           int nblocks) {
+  __shared__ unsigned s_count[2][32];
+  const bool counts = ((unsigned)block * 2654435761u >> 16) % (unsigned)(nblocks / 48 + 1) == 0u;
+  if (counts) {
+    if (threadIdx.x < 64) s_count[threadIdx.x >> 5][threadIdx.x & 31] = 0u;
+    __syncthreads();
+  }
   const int oct = F.U / 8;
+  const int64_t i = (int64_t)block * kSplitBlock + threadIdx.x;
   const int o = (int)(i % oct);
-  const int64_t col = i / oct;  // unit, angle and column
-  const int64_t per_unit = (int64_t)P4 * F.RP;
-  const int unit = first + (int)(col / per_unit);
-  const int64_t e = (int64_t)(unit % F.ring) * F.unit_elems + col % per_unit * F.U + o * 8;
-  const Vec<8> v = load_vec<8>(reinterpret_cast<const float*>(F.base) + e);
-  Vec<8> hi, lo;
+  const int64_t e = (int64_t)(unit % F.ring) * F.unit_elems + i * 8;  // column i / oct
+  const bool in = i < (int64_t)P4 * F.RP * oct;
+  Vec<8> x;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) x.v[j] = 0.f;
+  if (in) {
+    x = load_vec<8>(reinterpret_cast<const float*>(F.base) + e);
+    Vec<8> hi, lo;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int s = unit * F.U + o * 8 + j;
+      x.v[j] *= s < S ? split_scale(F.stat[s].most) : 1.f;
+      hi.v[j] = __half2float(__float2half_rn(x.v[j]));
+      lo.v[j] = fsub(x.v[j], hi.v[j]);
+    }
+    __half* dst = F.split + (e - o * 8) * 2 + o * 8;
+    store_hvec<8>(dst, hi);
+    store_hvec<8>(dst + F.U, lo);
+  }
+  if (!counts) return;
+  // the warp's lanes of the same 8 slices
+  const unsigned same = (oct == 4 ? 0x11111111u : oct == 2 ? 0x55555555u : ~0u) << o;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const int s = unit * F.U + o * 8 + j;
-    const float x = v.v[j] * (s < S ? split_scale(F.stat[s].most) : 1.f);
-    hi.v[j] = __half2float(__float2half_rn(x));
-    lo.v[j] = fsub(x, hi.v[j]);
+    const bool some = x.v[j] != 0.f;
+    const unsigned n = __popc(__ballot_sync(0xffffffffu, some) & same);
+    const unsigned m = __popc(__ballot_sync(0xffffffffu, some && fabsf(x.v[j]) < 0.5f) & same);
+    if ((threadIdx.x & 31) < oct) {
+      if (n) atomicAdd(&s_count[0][o * 8 + j], n);
+      if (m) atomicAdd(&s_count[1][o * 8 + j], m);
+    }
   }
-  __half* dst = F.split + (e - o * 8) * 2 + o * 8;
-  store_hvec<8>(dst, hi);
-  store_hvec<8>(dst + F.U, lo);
+  __syncthreads();
+  const int s = unit * F.U + threadIdx.x;
+  if (threadIdx.x < F.U && s < S) {
+    if (s_count[0][threadIdx.x]) atomicAdd(&F.stat[s].nonzero, s_count[0][threadIdx.x]);
+    if (s_count[1][threadIdx.x]) atomicAdd(&F.stat[s].small, s_count[1][threadIdx.x]);
+  }
 }
 
-__global__ void k_split_factors(const __grid_constant__ FactorDev F, int P4, int S, int first,
-                                int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) split_factors(F, P4, S, first, i);
+__global__ void __launch_bounds__(kSplitBlock)
+    k_split_factors(const __grid_constant__ FactorDev F, int P4, int S, int first) {
+  split_unit(F, P4, S, first + blockIdx.y, blockIdx.x, gridDim.x);
 }
 
-__global__ void k_split_factors_multi(const FinItem* __restrict__ items, int nitems) {
+__global__ void __launch_bounds__(kSplitBlock)
+    k_split_factors_multi(const FinItem* __restrict__ items, int nitems) {
   const FinItem& it = items[item_of(items, nitems, blockIdx.x)];
-  const int64_t i = (int64_t)(blockIdx.x - it.first) * blockDim.x + threadIdx.x;
-  if (i < it.nrays) split_factors(it.F, it.P4, it.S, 0, i);
+  const int b = (int)(blockIdx.x - it.first), per = (int)it.nrays;
+  split_unit(it.F, it.P4, it.S, b / per, b % per, per);
 }
 
 template <int K, bool FH>
@@ -967,18 +1001,15 @@ void launch_fwd_finish_units(const IterArgs& A, const TileMatrixDev& T, const fl
   }
 }
 
-static int64_t split_count(const FactorDev& F, int P4, int nunits) {
-  return (int64_t)nunits * P4 * F.RP * (F.U / 8);
-}
-int64_t split_blocks(const FactorDev& F, int P4, int nunits) {
-  return (split_count(F, P4, nunits) + 255) / 256;
+int64_t split_blocks(const FactorDev& F, int P4) {
+  return ((int64_t)P4 * F.RP * (F.U / 8) + kSplitBlock - 1) / kSplitBlock;
 }
 void launch_split_factors(const IterArgs& A, int first, int nunits, cudaStream_t st) {
-  const int64_t n = split_count(A.F, A.M.P4, nunits);
-  k_split_factors<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(A.F, A.M.P4, A.S, first, n);
+  k_split_factors<<<dim3((unsigned)split_blocks(A.F, A.M.P4), (unsigned)nunits), kSplitBlock, 0,
+                    st>>>(A.F, A.M.P4, A.S, first);
 }
 void launch_split_factors_multi(const FinItem* items, int n, int64_t blocks, cudaStream_t st) {
-  k_split_factors_multi<<<(unsigned)blocks, 256, 0, st>>>(items, n);
+  k_split_factors_multi<<<(unsigned)blocks, kSplitBlock, 0, st>>>(items, n);
 }
 
 template <int K, int LK, bool H, bool COMP>
