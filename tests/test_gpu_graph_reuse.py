@@ -37,3 +37,29 @@ def test_resets_between_captured_passes(size, kw):
         assert np.array_equal(bits(got[0]), bits(got[1])), (alg, beta, n, k)
     for plan in plans:
         plan.close()
+
+
+@pytest.mark.parametrize("K,S", [(8, 19), (16, 40), (4, 21)])
+def test_short_passes_before_and_after_their_capture(K, S):
+    """Short iterations on two streams are launched one by one at first (16 of
+    them) and captured then: every count of iterations gives the bits of plain
+    launches, across parameters that change and a reset that starts again."""
+    C, P = 48, 36
+    kw = dict(mode="fast", len_storage="u16", delta_index=True, forward_tiles=True,
+              half_gathers=True, slices_per_pass=K)
+    sino = np.random.default_rng(1).uniform(5.0, 9.0, (P, S, C)).astype(np.float32)
+    plans = [tg.Plan(P, S, C, theta_uniform(P), **kw) for _ in range(2)]
+    plans[0].set_graphs(True)
+    for plan in plans:
+        plan.set_sinogram(sino, apply_abs=True)
+    for again in range(2):
+        for plan in plans:
+            plan.reset_recon("pml")
+        for n, beta in ((15, 0.1), (1, 0.1), (1, 0.1), (4, 0.1), (3, 0.3), (2, 0.1)):
+            got = []
+            for plan in plans:
+                plan.iterate("pml", n, tg.default_params("pml", beta=beta))
+                got.append(plan.get_recon("pml"))
+            assert np.array_equal(bits(got[0]), bits(got[1])), (again, n, beta)
+    for plan in plans:
+        plan.close()

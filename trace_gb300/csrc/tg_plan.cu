@@ -124,6 +124,7 @@ struct tg_plan {
     tg_params prm{};
     cudaGraphExec_t exec = nullptr;
   } graphs[2];
+  int uncaptured = 0;  // iterations launched one by one since they were dropped
   // device address of the allocation-free entry point's factor array in the
   // context this plan was created in (looked up at creation), or nullptr
   float* noalloc_factors = nullptr;
@@ -371,21 +372,31 @@ void drop_graphs(tg_plan* p) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
     g = tg_plan::Graph();
   }
+  p->uncaptured = 0;
 }
 
-// Whether captured iterations are worth two branches, and outlive a reset of the
-// reconstruction whose buffers stay. A graph of two branches takes the host some
-// 60 us to launch, and destroying a graph that still runs waits for it. For long
-// iterations the branches fill each other's tails and the wait is what costs
-// (725 columns, 411 angles, 13 slices, 2 MLEM iterations: 1.83 ms a pass among
-// others and 1.95 alone; 1.97 and 1.98 captured anew each pass; 1.83 and 2.14 on
-// one branch). For short ones the launch costs more than it hides (67 columns,
-// 45 angles, 14 slices, 3 APMLR iterations: 107 us on one branch, 208 on two),
-// and the wait keeps the host from filling the GPU's launch queue (128 columns,
-// one slice, 10 iterations, 3000 passes ahead: 140 us a pass, 690 without).
-// The line is about 0.25 ms an iteration. (The scalar kernels' two chains have
-// nothing to wait for but their end: two branches always.)
+// Whether captured iterations outlive a reset of the reconstruction whose buffers
+// stay: destroying a graph that still runs waits for it. For long iterations that
+// wait is what costs (725 columns, 411 angles, 13 slices, 2 MLEM iterations: 1.83
+// ms a pass among others and 1.95 alone; 1.97 and 1.98 captured anew each pass);
+// for short ones it keeps the host from filling the GPU's launch queue (128 columns,
+// one slice, 10 iterations, 3000 passes ahead: 140 us a pass, 690 without). The
+// line is about 0.25 ms an iteration.
 bool long_pass(const tg_plan* p) { return p->g2 * p->P * p->S >= 500000000; }
+
+// Whether an iteration of a plan with the tensor-core backprojection has work for
+// two streams: more than one forward launch. On small grids a launch leaves most
+// of the GPU to the other stream's (a captured iteration of 64 columns, 48 angles,
+// 16 slices: 49.5 us on one branch, 32.1 on two; 256 columns, 180 angles: 107 and
+// 89).
+bool has_two_chains(const tg_plan* p) { return p->two && p->nb > p->forward_nb; }
+
+// Iterations of a short pass on two streams that are launched one by one before
+// they are captured: two branches take the host several of them to capture and
+// instantiate, which short reconstructions, whose graphs a reset drops, would pay
+// each time (67 columns, 45 angles, 14 slices, reset and 3 APMLR iterations: 153 us
+// a pass, 220 captured at once, on one branch).
+constexpr int kUncaptured = 16;
 
 int establish_layout(tg_plan* p, int alg) {
   if (!valid_alg(alg)) return fail(p, TG_E_ARG, "unknown algorithm");
@@ -1795,12 +1806,21 @@ int tg_iterate(tg_plan* p, int alg, const tg_params* prm, int n_iter) {
     if (graphs) {
       tg_plan::Graph& g = p->graphs[p->cur];
       const int hf = half_factors_next(p, mode);
-      if (!g.valid || g.alg != alg || g.half_factors != hf || !same_params(g.prm, prm)) {
+      const bool fits =
+          g.valid && g.alg == alg && g.half_factors == hf && same_params(g.prm, prm);
+      if (!fits && p->mma && !long_pass(p) && has_two_chains(p) && p->uncaptured < kUncaptured) {
+        issue_iteration(p, A, mode, true);
+        ++p->uncaptured;
+        p->cur ^= 1;
+        ++p->iters_done;
+        continue;
+      }
+      if (!fits) {
         if (g.exec) cudaGraphExecDestroy(g.exec);
         g = tg_plan::Graph();
         cudaGraph_t graph;
         TG_CUDA(p, cudaStreamBeginCapture(p->st, cudaStreamCaptureModeThreadLocal));
-        issue_iteration(p, A, mode, !p->mma || long_pass(p));
+        issue_iteration(p, A, mode, !p->mma || has_two_chains(p));
         TG_CUDA(p, cudaStreamEndCapture(p->st, &graph));
         const cudaError_t e = cudaGraphInstantiate(&g.exec, graph, 0);
         cudaGraphDestroy(graph);
