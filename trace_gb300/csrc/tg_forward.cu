@@ -74,7 +74,10 @@ __global__ void __launch_bounds__(kBlock)
     k_forward(DevGeom G, MatrixDev M, int ngroups,
               const float* __restrict__ recon, const float* __restrict__ sino,
               float* __restrict__ out, int out_mode) {
-  const int grp = (batch_block<K>(G, recon, sino, out) * kBlock + threadIdx.x) >> 5;
+  // 16 slices per pass: always a single batch (its pointers cost registers: 128
+  // columns, 90 angles, 24 exact slices 0.32 ms an iteration, 0.38 with them)
+  const int block = K == 16 ? (int)blockIdx.x : batch_block<K>(G, recon, sino, out);
+  const int grp = (block * kBlock + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (grp >= ngroups) return;  // warp-uniform
   const int a = grp / G.gpa;
@@ -345,7 +348,8 @@ template <int K, int LK>
 void fwd_launch(const IterArgs& A, int nb, const float* recon, const float* sino,
                 float* out, int out_mode, cudaStream_t st) {
   const int ngroups = A.G.P * A.G.gpa;
-  const dim3 blocks = batch_grid(((int64_t)ngroups * 32 + kBlock - 1) / kBlock, nb);
+  const int64_t all = ((int64_t)ngroups * 32 + kBlock - 1) / kBlock;
+  const dim3 blocks = K == 16 ? dim3((unsigned)all) : batch_grid(all, nb);
 #define TG_FWD(E, D) \
   k_forward<K, LK, E, D><<<blocks, kBlock, 0, st>>>(A.G, A.M, ngroups, recon, sino, out, out_mode)
   if (A.delta_index) {
