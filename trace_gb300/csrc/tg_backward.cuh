@@ -1,6 +1,6 @@
 // Backprojection (pixel-driven) with the algorithms' UpdateRecon fused into
 // its epilogue: exact mode, plans without the tile-staged forward, few slices,
-// fewer than 8 slices per pass with FP32 operands, compensated sums and the
+// FP32 operands at few slices per unit, compensated sums and the
 // allocation-free entry point. The other plans' runs on the tensor cores
 // (tg_backward_mma.cuh); one slice per pass without compensated sums is
 // tg_backward_planes.cu's.
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(kBlock, (min_blocks<K, COMP>()))
 
 // Multi-plan launches for plans with 16-bit fixed-point lengths (backward
 // matrix u16 codes, or IEEE halves with half gathers): compensated sums, few
-// slices, or FP32 operands at fewer than 8 slices per pass; the rest is
+// slices, or FP32 operands at few slices per unit; the rest is
 // tg_backward_mma.cuh's.
 template <int K>
 void back_multi(const BackItem* items, int n, int64_t blocks, int dlen_kind, int pen,
@@ -446,7 +446,7 @@ void back_multi(const BackItem* items, int n, int64_t blocks, int dlen_kind, int
       if (fh) TG_BM(LK_F16, true, false); else TG_BM(LK_F16, false, false);
     }
   } else if (!comp) {
-    if constexpr (K < 8) TG_BM(LK_U16, false, false);
+    TG_BM(LK_U16, false, false);
   } else if (dlen_kind == LK_F16) {
     if (fh) TG_BM(LK_F16, true, true); else TG_BM(LK_F16, false, true);
   } else {

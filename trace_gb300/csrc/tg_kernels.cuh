@@ -499,7 +499,7 @@ void launch_forward_tiled_multi(const FwdItem* items, int n, int64_t blocks, int
 void launch_fwd_finish_multi(const FinItem* items, int n, int64_t blocks, int K, int comp,
                              cudaStream_t st);
 // plans with 16-bit fixed-point lengths (backward matrix u16, or f16 with
-// half gathers), compensated or with FP32 operands at K < 8; pen: PML/APMLR;
+// half gathers), compensated or of few slices per unit; pen: PML/APMLR;
 // fh: half factors
 void launch_backward_multi(const BackItem* items, int n, int64_t blocks, int K,
                            int dlen_kind, int pen, int fh, int comp, cudaStream_t st);

@@ -1290,10 +1290,9 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
   p->info.window_exceptions = (int64_t)nexc;
   (void)counters[1];
   // The backprojection runs on the tensor cores for half-gather plans with
-  // 16-bit lengths (f16 in the backward matrix), and for FP32 operands at 8
-  // slices per pass or where a unit serves several passes (768 x 768, 540 angles,
-  // 16 slices, 2 PML iterations: 8 per pass 6.8 ms scalar and 5.6, 4 per pass 7.9
-  // and 6.2). A larger unit of slices spreads a tile's A operand over
+  // 16-bit lengths (f16 in the backward matrix), and for FP32 operands where a unit
+  // serves several passes (768 x 768, 540 angles, 16 slices, 2 PML iterations: 8
+  // per pass 6.8 ms scalar and 5.6, 4 per pass 7.9 and 6.2). A larger unit of slices spreads a tile's A operand over
   // more slices (1024 x 1024, 720 angles, per 8 slices: 0.96 ms in units of 8,
   // 0.61 of 16, 0.39 of 32), but a small grid has too few blocks to fill the
   // GPU with, so the unit is the largest one that leaves two blocks per SM.
@@ -1312,7 +1311,19 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     while (U > 8 && mma_regions(C) * ((p->S + U - 1) / U) < 2 * sms) U /= 2;
-    if (!d.half_gathers && p->K < 8) p->mma = U > p->K && p->S > 4;
+    // FP32 operands: fewer than 8 slices per pass and at most 4 slices keep the
+    // scalar kernels. A single unit of 8 slices serves but one pass of 8, or two of
+    // 4; f16 lengths are faster there all the same (900 columns, 600 angles, 8 per
+    // pass: 2.48 ms an iteration scalar, 1.94), the others' TF32 parts only while the
+    // blocks are one wave (8 per pass, u16: 260 columns 125 us scalar, 119; 300 columns
+    // 142 and 152; 900 2.45 ms and 2.94; f32 138 us and 127, 161 and 154, 2.78 ms and
+    // 2.99), or three blocks per SM against two launches (4 per pass, f32: 240 columns
+    // 106 us and 101, 260 118 and 123, 420 351 and 383).
+    if (!d.half_gathers) {
+      if (p->K < 8) p->mma = U > p->K && p->S > 4;
+      if (p->S <= 8 && p->K >= 4 && M.dlen_kind != LK_F16)
+        p->mma = p->mma && mma_regions(C) <= (p->K == 8 ? 4 : 3) * sms;
+    }
   }
   if (p->mma) {
     p->unit = std::max(U, p->K);
@@ -1322,7 +1333,12 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
     // takes 8 of them at once all the same, and reads the tile stream once for
     // them (forward and finish, 1024 x 1024, 720 angles, 16 slices in passes of
     // 4: 2.2 ms, 3.1 pass by pass; 256 x 256, 180 angles, 8 slices: 0.050, 0.071).
-    if (d.half_gathers && p->K < 8 && p->nb >= 8 / p->K) p->forward_nb = 8 / p->K;
+    // Two passes of 4 alone are faster side by side on the two streams while a
+    // launch leaves most of the GPU idle (8 slices, MLEM iteration: 128 columns 30 us
+    // and 35 at once, 160 36 and 41, 200 50.5 and 49.4, 256 69 and 67).
+    if (d.half_gathers && p->K < 8 && p->nb >= 8 / p->K &&
+        !(p->K == 4 && p->nb == 2 && C < 192 && d.batch_streams != 1))
+      p->forward_nb = 8 / p->K;
     M.tiles4 = (C + 3) / 4;
     uint32_t* place = nullptr;
     if ((rc = dalloc(p, &place, (size_t)M.tiles4 * M.tiles4 * 16 * (P4 / 4)))) return bail(rc);
