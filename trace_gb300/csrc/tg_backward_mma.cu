@@ -6,6 +6,7 @@
 namespace tg {
 
 TG_MMA_ENTRY(half, LK_F16, FK_HALF, 1)
+TG_MMA_MULTI_ENTRY(half, LK_F16, FK_HALF, 1)
 
 void launch_backward_mma(const IterArgs& A, int first, int nunits, const float* cur,
                          float* next, float* rep, int epi, cudaStream_t st) {

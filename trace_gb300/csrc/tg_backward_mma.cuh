@@ -811,7 +811,9 @@ void mma_multi(const BackItem* items, int n, int64_t blocks, int pen, cudaStream
 }  // namespace
 
 // Launches of one kind of factors and lengths, each in its own translation
-// unit (tg_backward_mma_*.cu) so that the instances build in parallel.
+// unit (tg_backward_mma_*.cu) so that the instances build in parallel; the
+// multi-plan launches (TG_MMA_MULTI_ENTRY) serve plans with 16-bit fixed-point
+// lengths.
 #define TG_MMA_ENTRY(KIND, LK, FK, LP)                                                      \
   void launch_backward_mma_##KIND(const IterArgs& A, int first, int nunits,                \
                                   const float* recon_cur, float* recon_next,               \
@@ -822,7 +824,8 @@ void mma_multi(const BackItem* items, int n, int64_t blocks, int pen, cudaStream
       mma_launch<2, LK, FK, LP>(A, first, nunits, recon_cur, recon_next, rep_num, epi, st); \
     else                                                                                    \
       mma_launch<4, LK, FK, LP>(A, first, nunits, recon_cur, recon_next, rep_num, epi, st); \
-  }                                                                                         \
+  }
+#define TG_MMA_MULTI_ENTRY(KIND, LK, FK, LP)                                                \
   void launch_backward_mma_multi_##KIND(const BackItem* items, int n, int64_t blocks,      \
                                         int U, int pen, cudaStream_t st) {                 \
     if (U == 8)                                                                             \

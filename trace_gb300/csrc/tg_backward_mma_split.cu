@@ -5,5 +5,6 @@
 namespace tg {
 
 TG_MMA_ENTRY(split, LK_F16, FK_SPLIT, 1)
+TG_MMA_MULTI_ENTRY(split, LK_F16, FK_SPLIT, 1)
 
 }  // namespace tg

@@ -5,5 +5,6 @@
 namespace tg {
 
 TG_MMA_ENTRY(u16, LK_U16, FK_TF32, 2)
+TG_MMA_MULTI_ENTRY(u16, LK_U16, FK_TF32, 2)
 
 }  // namespace tg

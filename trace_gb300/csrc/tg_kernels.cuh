@@ -404,7 +404,8 @@ void launch_backward_mma_multi(const BackItem* items, int n, int64_t blocks, int
 #define TG_MMA_DECL(KIND)                                                                  \
   void launch_backward_mma_##KIND(const IterArgs& A, int first, int nunits,               \
                                   const float* recon_cur, float* recon_next,              \
-                                  float* rep_num, int epi, cudaStream_t st);              \
+                                  float* rep_num, int epi, cudaStream_t st);
+#define TG_MMA_MULTI_DECL(KIND)                                                            \
   void launch_backward_mma_multi_##KIND(const BackItem* items, int n, int64_t blocks,     \
                                         int U, int pen, cudaStream_t st);
 TG_MMA_DECL(half)
@@ -412,6 +413,10 @@ TG_MMA_DECL(split)
 TG_MMA_DECL(u16)
 TG_MMA_DECL(bf16)
 TG_MMA_DECL(f32)
+TG_MMA_MULTI_DECL(half)
+TG_MMA_MULTI_DECL(split)
+TG_MMA_MULTI_DECL(u16)
+#undef TG_MMA_MULTI_DECL
 #undef TG_MMA_DECL
 // tg_backward_staged.cu (fast mode)
 void launch_backward_staged(const IterArgs& A, int batch, const float* recon_cur,
