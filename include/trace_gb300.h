@@ -182,7 +182,8 @@ typedef struct {
   int64_t num_segments;       /* traced ray-pixel segments (one slice) */
   int64_t forward_bytes;      /* bytes of the forward (ray-major) matrix */
   int64_t backward_bytes;     /* bytes of the backward (pixel-major) matrix */
-  int64_t device_bytes;       /* all device memory held by the plan */
+  int64_t device_bytes;       /* all device memory held by the plan, with the
+                                 unused ends of its chunks */
   float max_segment_length;
   double setup_ms;            /* time spent tracing and building matrices */
   int batches;                /* ceil(stored slices / slices_per_pass) */

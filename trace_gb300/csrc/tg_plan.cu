@@ -183,6 +183,7 @@ int dalloc(tg_plan* p, T** out, size_t count, bool zero = false, bool own = fals
     if (c == p->chunks.end()) {
       void* base = nullptr;
       if (cudaMalloc(&base, p->chunk) == cudaSuccess) {
+        p->dev_bytes += (int64_t)p->chunk;
         p->chunks.push_back({static_cast<char*>(base), p->chunk, 0});
         c = p->chunks.end() - 1;
       } else {
@@ -203,8 +204,8 @@ int dalloc(tg_plan* p, T** out, size_t count, bool zero = false, bool own = fals
                       cudaGetErrorString(e));
     }
     p->allocs.push_back(ptr);
+    p->dev_bytes += (int64_t)bytes;
   }
-  p->dev_bytes += (int64_t)bytes;
   if (zero) {
     e = cudaMemsetAsync(ptr, 0, bytes, p->st);
     if (e != cudaSuccess) return fail(p, TG_E_CUDA, cudaGetErrorString(e));
@@ -214,12 +215,12 @@ int dalloc(tg_plan* p, T** out, size_t count, bool zero = false, bool own = fals
 }
 
 // A chunk takes back only its last buffer, and only while the plan is made
-// (everything runs on one stream then).
+// (everything runs on one stream then): temporaries are freed last one first.
 void dfree(tg_plan* p, void* ptr, size_t bytes) {
   if (!ptr) return;
-  p->dev_bytes -= (int64_t)bytes;
   for (auto& a : p->allocs)
     if (a == ptr) {
+      p->dev_bytes -= (int64_t)bytes;
       a = nullptr;
       cudaFree(ptr);
       return;
@@ -489,7 +490,7 @@ int build_tiles(tg_plan* p, int* d_nruns) {
     return rc;
   };
   auto release = [&]() {
-    for (auto& t : tmp) dfree(p, t.first, t.second);
+    for (size_t i = tmp.size(); i-- > 0;) dfree(p, tmp[i].first, tmp[i].second);
     tmp.clear();
   };
   int rc = TG_OK;
@@ -727,7 +728,7 @@ int build_strips(tg_plan* p, const StripTables& T) {
   std::vector<void*> got;  // kept allocations, freed when the build gives up
   std::vector<size_t> size;
   auto give_up = [&]() {
-    for (size_t i = 0; i < got.size(); ++i) dfree(p, got[i], size[i]);
+    for (size_t i = got.size(); i-- > 0;) dfree(p, got[i], size[i]);
     p->d_simg = nullptr;
     p->d_spart = nullptr;
     p->err.clear();
@@ -780,8 +781,8 @@ int build_strips(tg_plan* p, const StripTables& T) {
       !keep(&meta, nsteps * 16, false) ||
       !keep(&p->d_simg, U * p->g2, false) || !keep(&p->d_spart, U * S.nbundles * 16, false))
     return give_up();
-  if (dalloc(p, &exc, kCap) != TG_OK) return give_up();
-  if (dalloc(p, &nexc, 1, true) != TG_OK) {
+  if (dalloc(p, &exc, kCap, false, true) != TG_OK) return give_up();
+  if (dalloc(p, &nexc, 1, true, true) != TG_OK) {
     dfree(p, exc, kCap * sizeof(StripExc));
     return give_up();
   }
@@ -813,7 +814,8 @@ int build_strips(tg_plan* p, const StripTables& T) {
   uint16_t* rlen = nullptr;
   bool ok = true;
   if (!M.rlen) {
-    ok = dalloc(p, &ridx, (size_t)T.entries) == TG_OK && dalloc(p, &rlen, (size_t)T.entries) == TG_OK;
+    ok = dalloc(p, &ridx, (size_t)T.entries, false, true) == TG_OK &&
+         dalloc(p, &rlen, (size_t)T.entries, false, true) == TG_OK;
     if (ok) launch_strips_trace(p->G, M, ridx, rlen, p->st);
     M.ridx = ridx;
     M.rlen = rlen;
@@ -1269,8 +1271,8 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
     M.exc_first = p->d_exc_first;
     M.exc = p->d_exc;
   }
-  dfree(p, d_exc_tmp, (size_t)kExcCap * sizeof(int4));
   dfree(p, d_exc_tile_tmp, (size_t)kExcCap * sizeof(int));
+  dfree(p, d_exc_tmp, (size_t)kExcCap * sizeof(int4));
   if (counters[0] && d.delta_index && !otf) {
     // a stray segment's step does not fit the 4-bit code: this plan's
     // ray-ordered forward projection traces its rays on the fly instead
