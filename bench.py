@@ -437,9 +437,9 @@ def _run_ours(args, W, ws, rank, local, dev, stream, tg, torch, np):
     t0 = time.time()
     tuned = None
     if args.autotune:
-        from trace_gb300.autotune import autotune
+        from trace_gb300.autotune import DEFAULT_SPACE, autotune
         from trace_gb300.phantom import ellipse_phantoms_torch
-        n = min(16, S)
+        n = min(32, S)  # the strip-ordered forward starts at 32 slices
         tp = tg.Plan(P, n, C, theta, len_storage=args.len_storage, mode="fast",
                      delta_index=True)
         tp.set_stream(stream)
@@ -448,8 +448,10 @@ def _run_ours(args, W, ws, rank, local, dev, stream, tg, torch, np):
         sample = torch.empty((P, n, C), dtype=torch.float32, device=dev)
         tp.forward_project("sirt", out=sample)
         tp.close()
+        # the FP32 arms run at the same slices per pass, and 16 in tiles need half
+        # gathers
         best, res = autotune(theta, sample, alg, prm, len_storage=args.len_storage,
-                             stream=stream,
+                             stream=stream, space={**DEFAULT_SPACE, "slices_per_pass": (4, 8)},
                              fixed={"half_gathers": True} if args.half else None)
         K, args.tiles, args.staged = (best["slices_per_pass"], best["forward_tiles"],
                                       best["backward_staged"])
@@ -513,8 +515,9 @@ def _run_ours(args, W, ws, rank, local, dev, stream, tg, torch, np):
     dom = "backward" if tim["backward_ms"] >= tim["forward_ms"] else "forward"
     kf, kb = kernel_names(info, args, W, K, nb, per_step)
     kname = {"forward": kf, "backward": kb}[dom]
-    # the strips' forward is three launches (reset, halves, sums), the tensor-core
-    # backprojection of SIRT's float factors two (their halves first)
+    # the strips' forward is two launches (halves, sums) and so is their finish
+    # (values, walked slices), and the tensor-core backprojection of SIRT's float
+    # factors (their halves first)
     launches = round(args.steps * (sum(per_step.values()) if args.tiles
                                    else per_step["forward"] + per_step["backward"]))
     if kf == "k_forward_strips":

@@ -16,7 +16,9 @@ forward matrix) earns its place.
 The search is the full product of DEFAULT_SPACE (schedule choices that
 interact), then one dimension of REFINE_SPACE at a time from the best so far
 (tile side and tile shape are independent refinements of the kernels the
-schedule picked).
+schedule picked; a plan with the strip-ordered forward reads neither tile sides
+nor block warps). A plan's kernels depend on its slices - half-gather plans take
+the strips from 32 on -, so the sample should have as many as the plan, or 32.
 """
 from __future__ import annotations
 
@@ -48,8 +50,8 @@ TG_E_NOMEM = 3
 
 def _measure(theta, sino, alg, params, len_storage, cfg, fixed, iters, warmup, stream,
              max_device_bytes):
-    """(ms per slice-iteration, setup ms, device bytes) of one configuration;
-    None if the plan rejects the combination."""
+    """(ms per slice-iteration, setup ms, device bytes, strip-ordered forward)
+    of one configuration; None if the plan rejects the combination."""
     P, S, C = (int(x) for x in sino.shape)
     t0 = time.perf_counter()
     try:
@@ -60,12 +62,15 @@ def _measure(theta, sino, alg, params, len_storage, cfg, fixed, iters, warmup, s
             return None  # not a valid combination (e.g. half_gathers + staged)
         if e.status != TG_E_NOMEM:
             raise
-        return math.inf, 0.0, None
+        return math.inf, 0.0, None, False
     setup_ms = (time.perf_counter() - t0) * 1e3
-    nbytes = plan.info()["device_bytes"]
+    info = plan.info()
+    nbytes = info["device_bytes"]
+    # the strips count one run per ray and chunk of rows
+    strips = info["tile_runs"] > 0 and info["tile_runs"] % (P * C) == 0
     if max_device_bytes is not None and nbytes > max_device_bytes:
         plan.close()
-        return math.inf, setup_ms, nbytes
+        return math.inf, setup_ms, nbytes, strips
     if stream is not None:
         plan.set_stream(stream)
     plan.set_sinogram(sino, apply_abs=alg != "sirt")
@@ -77,7 +82,7 @@ def _measure(theta, sino, alg, params, len_storage, cfg, fixed, iters, warmup, s
     plan.synchronize()
     ms = (time.perf_counter() - t1) * 1e3 / (iters * S)
     plan.close()
-    return ms, setup_ms, nbytes
+    return ms, setup_ms, nbytes, strips
 
 
 def autotune(theta, sino, alg="pml", params=None, *, len_storage="u16",
@@ -98,13 +103,16 @@ def autotune(theta, sino, alg="pml", params=None, *, len_storage="u16",
     refine = REFINE_SPACE if refine is None else refine
     params = params or default_params(alg)
     results = []
+    on_strips = []  # configurations whose plans have the strip-ordered forward
 
     def run(cfg):
         r = _measure(theta, sino, alg, params, len_storage, cfg, fixed, iters, warmup,
                      stream, max_device_bytes)
         if r is None:
             return None
-        results.append((dict(cfg), *r))
+        results.append((dict(cfg), *r[:3]))
+        if r[3]:
+            on_strips.append(dict(cfg))
         if log:
             log(f"autotune {cfg}: {r[0]:.3f} ms per slice-iteration")
         return r[0]
@@ -122,8 +130,8 @@ def autotune(theta, sino, alg="pml", params=None, *, len_storage="u16",
     best_cfg, best_ms = min(fitting, key=lambda r: r[1])[:2]
     best_cfg = dict(best_cfg)
     for key, values in refine.items():
-        if key in ("forward_tile_side", "forward_block_warps") and not best_cfg.get(
-                "forward_tiles"):
+        if key in ("forward_tile_side", "forward_block_warps") and (
+                not best_cfg.get("forward_tiles") or best_cfg in on_strips):
             continue
         for v in values:
             if key not in best_cfg and v == PLAN_DEFAULTS.get(key):
