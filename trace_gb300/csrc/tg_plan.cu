@@ -166,9 +166,12 @@ int fail(tg_plan* p, int code, const std::string& msg) {
 // what is at most half a chunk comes out of the plan's chunks, which live as
 // long as the plan (a 256 x 256 plan with 180 angles: 1680 us to make it
 // and 420 to destroy it, 2220 and 610 each buffer for itself). own: a buffer
-// that is freed or replaced while the plan lives, for itself.
+// that is freed or replaced while the plan lives, for itself. more: bytes that the
+// chunk should have left for the next calls' buffers (a new chunk takes some 50 us,
+// which an upload has and a first iteration feels).
 template <class T>
-int dalloc(tg_plan* p, T** out, size_t count, bool zero = false, bool own = false) {
+int dalloc(tg_plan* p, T** out, size_t count, bool zero = false, bool own = false,
+           size_t more = 0) {
   void* ptr = nullptr;
   const size_t bytes = count * sizeof(T);
   if (bytes == 0) {
@@ -179,7 +182,7 @@ int dalloc(tg_plan* p, T** out, size_t count, bool zero = false, bool own = fals
   const size_t room = (bytes + 511) / 512 * 512;
   if (!own && room <= p->chunk / 2) {
     auto c = std::find_if(p->chunks.begin(), p->chunks.end(),
-                          [&](const tg_plan::Chunk& k) { return k.size - k.used >= room; });
+                          [&](const tg_plan::Chunk& k) { return k.size - k.used >= room + more; });
     if (c == p->chunks.end()) {
       void* base = nullptr;
       if (cudaMalloc(&base, p->chunk) == cudaSuccess) {
@@ -1501,7 +1504,14 @@ static int set_sinogram(tg_plan* p, const float* sino, int on_device,
                         int apply_abs, int clip, float clip_min) {
   if (!p || !sino) return p ? fail(p, TG_E_ARG, "null sinogram") : TG_E_ARG;
   const size_t n = (size_t)p->P * p->S * p->C;
-  if (!p->d_sino) TG_TRY(dalloc(p, &p->d_sino, (size_t)p->nb * p->R * p->K));
+  if (!p->d_sino) {
+    // and the iterations' float factors with their halves
+    const size_t f = p->mma ? (size_t)std::min(p->nunits, 2 * p->group_units) * p->unit * p->M.P4 *
+                                  factor_row(p->C) * 8 + (1 << 16)
+                            : 0;
+    const size_t n = (size_t)p->nb * p->R * p->K;
+    TG_TRY(dalloc(p, &p->d_sino, n, false, false, n * 4 + f < p->chunk ? f : 0));
+  }
   TG_CUDA(p, cudaMemsetAsync(p->d_sino, 0,
                              (size_t)p->nb * p->R * p->K * sizeof(float), p->st));
   const float* src = sino;
