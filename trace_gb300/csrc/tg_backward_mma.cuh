@@ -375,6 +375,11 @@ __device__ __forceinline__ void backward_mma_block(const IterArgs& A, int unit, 
   const uint32_t* dl = reinterpret_cast<const uint32_t*>(A.M.dlen);
   const int64_t unit_base = (int64_t)(unit % A.F.ring) * A.F.unit_elems;
   const int P4 = A.M.P4, RP = A.F.RP;
+  // the slices that the products do not serve: looked up now or after the products,
+  // what suits the kernel's registers (PML, half factors, 2048 x 2048, 1500 angles, 64
+  // slices 26.4 ms, after them 27.1)
+  unsigned redo = 0u;
+  if constexpr (FK == FK_HALF) redo = redo_slices<false>(A, unit, lane);
 
   float acc[NT][4];
 #pragma unroll
@@ -616,7 +621,7 @@ __device__ __forceinline__ void backward_mma_block(const IterArgs& A, int unit, 
   // Slices that the products do not serve: their sums again, ray by ray, into shared
   // memory ([warp][16 pixels][U]; kept out of the accumulators' registers). A lane
   // takes one of the tile's 16 pixels and half of the angle quads.
-  const unsigned redo = redo_slices<FK == FK_SPLIT>(A, unit, lane);
+  if constexpr (FK != FK_HALF) redo = redo_slices<FK == FK_SPLIT>(A, unit, lane);
   float* const again = reinterpret_cast<float*>(sm) + warp * 16 * U;
   static_assert(kMmaTiles * 16 * U * 4 <= St::kBytes, "the sums fit the stages");
   if (redo) {

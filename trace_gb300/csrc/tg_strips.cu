@@ -26,8 +26,8 @@
 // The tile-staged forward (tg_tiles.cu) reads a 16-byte pixel vector from
 // shared memory per segment and 8 slices and is bound by those wavefronts
 // (94 %) and issue (77 %). 1024 x 1024, 720 angles, 64 slices: 7.8 ms there
-// with 0.4 for its finish, 4.0 and 0.84 here; 2048 x 2048, 1500 angles: 56 and
-// 3 there, 29.8 and 3.6 here. Here one block of 16 warps fills an SM (128
+// with 0.4 for its finish, 4.0 and 0.73 here; 2048 x 2048, 1500 angles: 56 and
+// 3 there, 29.8 and 3.0 here. Here one block of 16 warps fills an SM (128
 // registers a thread); tensor pipe 38 %, shared memory 59 %, DRAM 41 %, and the
 // rest waits: the stage's barrier and the chain ldmatrix - product - sum.
 //
