@@ -402,6 +402,16 @@ def format_bytes(info, W, K, tiles, half=False):
     return fwd, back
 
 
+# from the captures in profiles/
+LIMITED_BY = {
+    "k_forward_strips": "no unit full: tensor pipe in bursts between stage barriers "
+                        "(41 %), L1TEX 55 %, DRAM 41 %",
+    "k_backward_mma": "issue (63 %) and ALU (52 %) of the sparse operand, L1TEX 60 %",
+    "k_forward_tiled": "shared-memory wavefronts and issue",
+    "k_backward": "L1 data pipe",
+}
+
+
 def kernel_names(info, args, W, K, nb, per_step):
     """The forward and the backward kernel of the schedule that was timed."""
     if not args.tiles:
@@ -533,9 +543,11 @@ def _run_ours(args, W, ws, rank, local, dev, stream, tg, torch, np):
         return b / (ms / 1e3) / 1e9 if ms else None
 
     roofline = {
+        # "bound" names the peak that the fraction is of; what the kernel waits for
+        # is "limited_by"
         "bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
         "frac": achieved / hbm_peak, "peak_kind": f"{peak_kind} (burst copy)",
-        "traffic": traffic, "kernel": kname,
+        "traffic": traffic, "kernel": kname, "limited_by": LIMITED_BY.get(kname),
         # the same kernel's measured DRAM bytes (ncu, one launch of this
         # configuration) over its live launch time: what HBM actually moved
         "achieved_traffic": gbs(traffic, dom_ms) if traffic else None,
@@ -1093,7 +1105,7 @@ def main():
                     help="no stored ray-ordered forward matrix: rays traced during "
                          "forward projections")
     ap.add_argument("--no-autotune", dest="autotune", action="store_false",
-                    help="skip timing the plan configurations on a 16-slice sample "
+                    help="skip timing the plan configurations on a 32-slice sample "
                          "(run the defaults or the flags given)")
     ap.add_argument("--forward-tile-side", dest="fts", type=int, default=0,
                     help="forward tile side (32, 64, 96; 0 = the plan default)")

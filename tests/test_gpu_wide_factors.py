@@ -90,3 +90,32 @@ def test_hot_slices_leave_the_others_bits():
         plan.close()
     same = [s for s in range(S) if s not in HOT]
     assert np.array_equal(bits(outs[0][same]), bits(outs[1][same]))
+
+
+@pytest.mark.parametrize("kind", ["u16", "f32", "f16"])
+def test_finite_factors_at_the_top_of_the_range(kind):
+    """Ratios from 1e38 on, which rounding up could make infinite: their slices are
+    summed ray by ray as those with an infinite factor."""
+    C, P, S = 34, 40, 9
+    rng = np.random.default_rng(C)
+    tabs = O.angle_table(theta_uniform(P))
+    sino = O.forward(rng.uniform(0.5, 1.5, (S, C, C)).astype(np.float32), tabs)
+    counts, offs, idx, *_ = O.trace(C, tabs)
+    start = np.full((S, C, C), 0.05, np.float32)
+    sim = O.forward(start[:1], tabs)[:, 0]  # of the ratio's first projection
+    hit = np.zeros((S, C * C), bool)
+    for s, (a, c) in HOT.items():
+        c = min(c, 20)
+        assert 1.05e38 < 3e38 / sim[a, c] < 3.3e38, (s, sim[a, c])
+        sino[a, s, c] = 3e38
+        r = a * C + c
+        hit[s, idx[offs[r]:offs[r] + counts[r]]] = True
+    ref = O.run("mlem", sino, tables=tabs, n_iter=1, precision=O.F64, want_replica=True,
+                recon_in=start)
+    plan = tg.Plan(P, S, C, theta_uniform(P), **KINDS[kind])
+    plan.set_sinogram(sino, apply_abs=True)
+    plan.set_recon("mlem", start)
+    plan.reduce("mlem")
+    got = plan.get_replica("mlem").reshape(S, -1, 2)[..., 0]
+    _check(got, ref["replica"].reshape(S, -1, 2)[..., 0], hit, TOL[kind])
+    plan.close()

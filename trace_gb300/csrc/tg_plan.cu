@@ -784,8 +784,8 @@ int build_strips(tg_plan* p, const StripTables& T) {
       !keep(&meta, nsteps * 16, false) ||
       !keep(&p->d_simg, U * p->g2, false) || !keep(&p->d_spart, U * S.nbundles * 16, false))
     return give_up();
-  if (dalloc(p, &exc, kCap, false, true) != TG_OK) return give_up();
-  if (dalloc(p, &nexc, 1, true, true) != TG_OK) {
+  if (dalloc(p, &exc, kCap) != TG_OK) return give_up();
+  if (dalloc(p, &nexc, 1, true) != TG_OK) {
     dfree(p, exc, kCap * sizeof(StripExc));
     return give_up();
   }
@@ -851,8 +851,8 @@ int build_strips(tg_plan* p, const StripTables& T) {
       ok = false;
     }
   }
-  dfree(p, exc, kCap * sizeof(StripExc));
   dfree(p, nexc, sizeof(int));
+  dfree(p, exc, kCap * sizeof(StripExc));
   if (ridx) dfree(p, ridx, (size_t)T.entries * 4);
   if (rlen) dfree(p, rlen, (size_t)T.entries * 2);
   if (rc != TG_OK) return rc;
