@@ -1323,10 +1323,12 @@ int tg_plan_create(const tg_plan_desc* desc, const float* theta,
     // blocks are one wave (8 per pass, u16: 260 columns 125 us scalar, 119; 300 columns
     // 142 and 152; 900 2.45 ms and 2.94; f32 138 us and 127, 161 and 154, 2.78 ms and
     // 2.99), or three blocks per SM against two launches (4 per pass, f32: 240 columns
-    // 106 us and 101, 260 118 and 123, 420 351 and 383).
+    // 106 us and 101, 260 118 and 123, 420 351 and 383; bf16, whose lengths are one
+    // TF32 part, 900 columns 2.67 ms and 2.56: always).
     if (!d.half_gathers) {
       if (p->K < 8) p->mma = U > p->K && p->S > 4;
-      if (p->S <= 8 && p->K >= 4 && M.dlen_kind != LK_F16)
+      if (p->S <= 8 && p->K >= 4 && M.dlen_kind != LK_F16 &&
+          !(p->K == 4 && M.dlen_kind == LK_BF16))
         p->mma = p->mma && mma_regions(C) <= (p->K == 8 ? 4 : 3) * sms;
     }
   }
